@@ -211,77 +211,8 @@ __device__ __forceinline__ void op_relax_pass(const Geom& g, const BrickTable& b
     const double resid = relax_brick<NX, TH, CT>(sm, D, Corr<CT>::dphi1(st) + (size_t)b * P3, lt, c, v, sync);
     CT* sw = snap_wr + (size_t)b * stride;
 #pragma unroll
-    for (int r = 0; r < K; r++) relax_put<NX, CT>(D, sw, lt + r * TH, v[r]);
+    for (int r = 0; r < K; r++) relax_put<NX, CT>(D, sw, relax_index<NX, TH>(lt, r), v[r]);
     if (lt == 0) pres[b] = resid;
-}
-
-// op_relax_pass in mode 1 split in two, so that a pass can be computed
-// before the loop has decided whether it runs.  op_relax_spec computes it
-// from the current dphi and the snapshot snap_rd with nothing written to
-// global memory (the ghost faces go to the staged brick only, where the
-// sweeps leave them); op_relax_commit then writes what op_relax_pass
-// writes: the ghost faces and the relaxed interior to dphi, the first
-// interior layers to snap_wr, the sum to pres[b].  Same values as
-// op_relax_pass; called by every thread of a block of TH threads, with the
-// brick's shared memory untouched in between.
-template <typename CT, int K>
-struct RelaxSpec {
-    CT v[K];       // this thread's relaxed interior cells
-    double resid;  // the brick's last sweep sum
-};
-
-template <int NX, int TH, typename CT>
-__device__ __forceinline__ RelaxSpec<CT, NX * NX * NX / TH> op_relax_spec(const Geom& g, const BrickTable& bt,
-                                                                        const DevState& st, int b, const CT* snap_rd,
-                                                                        size_t stride, RelaxSmem<NX, CT>& sm) {
-    constexpr int P = NX + 2, P3 = P * P * P, F = NX * NX, K = NX * NX * NX / TH, G = (6 * F + TH - 1) / TH;
-    const CT* D = Corr<CT>::dphi(st) + (size_t)b * P3;
-    const int lt = threadIdx.x;
-    CT gv[G];
-    int gi[G];
-#pragma unroll
-    for (int r = 0; r < G; r++) {
-        const int q = lt + r * TH;
-        gi[r] = -1;
-        if (q < 6 * F) {
-            int face, t1, t2;
-            gi[r] = relax_ghost_cell<NX>(q, face, t1, t2);
-            gv[r] = ghost_dphi<NX, CT>(g, bt, st, snap_rd, stride, b, face, t1, t2);
-        }
-    }
-    relax_stage<NX, TH, CT>(sm, D, lt);
-    int c[K];
-    CT d1[K];
-    relax_cells<NX, TH, CT>(lt, Corr<CT>::dphi1(st) + (size_t)b * P3, c, d1);
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < G; r++)
-        if (gi[r] >= 0) {
-            sm.buf[0][gi[r]] = gv[r];
-            sm.buf[1][gi[r]] = gv[r];
-        }
-    __syncthreads();
-    RelaxSpec<CT, K> out;
-    out.resid = relax_sweeps<NX, TH, CT>(sm, lt, c, d1, out.v, BlockSync{});
-    return out;
-}
-
-template <int NX, int TH, typename CT>
-__device__ __forceinline__ void op_relax_commit(const DevState& st, int b, const RelaxSpec<CT, NX * NX * NX / TH>& r,
-                                                const RelaxSmem<NX, CT>& sm, CT* snap_wr, size_t stride,
-                                                double* pres) {
-    constexpr int P = NX + 2, P3 = P * P * P, F = NX * NX, K = NX * NX * NX / TH;
-    CT* D = Corr<CT>::dphi(st) + (size_t)b * P3;
-    const int lt = threadIdx.x;
-    for (int q = lt; q < 6 * F; q += TH) {
-        int face, t1, t2;
-        const int gi = relax_ghost_cell<NX>(q, face, t1, t2);
-        D[gi] = sm.buf[0][gi];
-    }
-    CT* sw = snap_wr + (size_t)b * stride;
-#pragma unroll
-    for (int q = 0; q < K; q++) relax_put<NX, CT>(D, sw, lt + q * TH, r.v[q]);
-    if (lt == 0) pres[b] = r.resid;
 }
 
 }  // namespace amr

@@ -439,7 +439,7 @@ struct Solver {
             for (int f = 0; f < 6; f++) sib |= a.bt.ftype[6 * b + f] == FACE_SIB ? 1u << f : 0u;
 #pragma unroll
             for (int r = 0; r < K; r++)
-                relax_layer_put_tagged<NX>(sw, threadIdx.x + r * TPB, float(res[c[r]]), seq, sib);
+                relax_layer_put_tagged<NX>(sw, relax_index<NX, TPB>(threadIdx.x, r), float(res[c[r]]), seq, sib);
             if (threadIdx.x == 0) {
                 // the FP64 sum as two tagged halves (pres buffer of this pass)
                 const int pp = (int)((pres - a.pres) / a.L.cap);
@@ -451,7 +451,8 @@ struct Solver {
         } else {
             CT* sw = reinterpret_cast<CT*>(a.snap) + (size_t)wpar * a.snap_half + (size_t)b * a.stride;
 #pragma unroll
-            for (int r = 0; r < K; r++) relax_layer_put<NX, CT>(sw, threadIdx.x + r * TPB, res[c[r]]);
+            for (int r = 0; r < K; r++)
+                relax_layer_put<NX, CT>(sw, relax_index<NX, TPB>(threadIdx.x, r), res[c[r]]);
             if (threadIdx.x == 0) pres[b] = resid;
             __syncthreads();
             if (threadIdx.x == 0)
@@ -543,7 +544,7 @@ struct Solver {
         ok = !__syncthreads_or(bad);
         if (!ok) return 0.0;
         int sw;
-        const double r = relax_sweeps_in<NX, TPB, CT>(x, y, &sm[0].red[0][0], threadIdx.x, c, d1, res, BlockSync{}, &sw);
+        const double r = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, c, d1, res, BlockSync{}, &sw);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             rsplit[4]++;
             rsplit[5] += sw;
@@ -764,7 +765,7 @@ struct Solver {
             if (bulk && !wait_staged()) return false;
             __syncthreads();
             CT* res;
-            const double rs = relax_sweeps_in<NX, TPB, CT>(x, y, &sm[0].red[0][0], threadIdx.x, c, d1, &res,
+            const double rs = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, c, d1, &res,
                                                            BlockSync{});
             const int i = res == x ? 0 : 1;
             if (j) ib1 = i;

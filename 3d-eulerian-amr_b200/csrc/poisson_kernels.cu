@@ -320,9 +320,14 @@ int launch_relax(const Geom& g, const DevState& st, const int* slots, int n, dou
         if (f32)
             launch_k(k_relax<12, float>, n, RelaxThreads<12>::value, sizeof(RelaxSmem<12, float>), s, g, st, slots,
                      out);
-        else
+        else {
+            // above the 48 KB a launch may take without asking; per launch,
+            // since the attribute belongs to the current device
+            cudaFuncSetAttribute((const void*)k_relax<12, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(RelaxSmem<12, double>));
             launch_k(k_relax<12, double>, n, RelaxThreads<12>::value, sizeof(RelaxSmem<12, double>), s, g, st, slots,
                      out);
+        }
     } else {
         return -1;
     }
