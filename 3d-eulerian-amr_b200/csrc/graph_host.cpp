@@ -42,6 +42,12 @@ using namespace amr;
 // entries per brick in one face-snapshot buffer: 6 faces of nx*nx
 inline size_t snap_stride(const amr_ctx* c) { return 6 * (size_t)c->geom.nx * c->geom.nx; }
 
+// tagged words per brick in one buffer of the persistent solve's snapshots:
+// an entry of the FP32 correction is one word, of the FP64 correction two
+inline size_t tsnap_words(const amr_ctx* c) {
+    return snap_stride(c) * (c->geom.precision == AMR_PREC_MIXED ? 1 : 2);
+}
+
 struct GraphState {
     Control* d_ctl = nullptr;
     Control* h_ctl = nullptr;  // pinned mirror
@@ -71,9 +77,8 @@ struct GraphState {
     double* d_pres3 = nullptr;
     double* d_pnest = nullptr;
     GridBarrier* d_bar = nullptr;
-    unsigned* d_rpub = nullptr;  // [cap] relaxation pass words of the persistent solve
-    unsigned long long* d_tsnap = nullptr;  // [2][cap][6][nx][nx] tagged face snapshots (FP32 correction)
-    unsigned long long* d_tpres = nullptr;  // [2][cap][2] tagged per-brick relaxation sums (FP32 correction)
+    unsigned long long* d_tsnap = nullptr;  // [2][cap][6][nx][nx] tagged face snapshots, tsnap_words words an entry
+    unsigned long long* d_tpres = nullptr;  // [2][cap][2] tagged per-brick relaxation sums
     cudaEvent_t ev_ps[2] = {nullptr, nullptr};  // around the last persistent launch
     double ps_ms_total = 0.0;                   // persistent launches of amr_graph_solve: device time, count
     long long ps_count = 0;
@@ -117,11 +122,8 @@ int ensure_state(amr_ctx* c) {
         CUDA_TRY(cudaMalloc(&g->d_pres3, sizeof(double) * 3 * (size_t)c->cap));
         CUDA_TRY(cudaMalloc(&g->d_pnest, sizeof(double) * (size_t)g->pnest_blocks * c->cap));
         CUDA_TRY(cudaMalloc(&g->d_bar, sizeof(GridBarrier)));
-        CUDA_TRY(cudaMalloc(&g->d_rpub, sizeof(unsigned) * (size_t)c->cap));
-        if (c->geom.precision == AMR_PREC_MIXED) {
-            CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * snap_stride(c) * (size_t)c->cap));
-            CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
-        }
+        CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap));
+        CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
         CUDA_TRY(cudaEventCreate(&g->ev_ps[0]));
         CUDA_TRY(cudaEventCreate(&g->ev_ps[1]));
     }
@@ -321,14 +323,10 @@ int rec_persistent(amr_ctx* c, cudaStream_t s, double tol) {
     a.snap_half = snap_stride(c) * (size_t)c->cap;
     a.bar = g->d_bar;
     CUDA_TRY(cudaMemsetAsync(g->d_bar, 0, sizeof(GridBarrier), s));
-    a.rpub = g->d_rpub;
-    CUDA_TRY(cudaMemsetAsync(g->d_rpub, 0, sizeof(unsigned) * (size_t)c->cap, s));
     a.tsnap = g->d_tsnap;
     a.tpres = g->d_tpres;
-    if (g->d_tsnap) {
-        CUDA_TRY(cudaMemsetAsync(g->d_tsnap, 0, sizeof(unsigned long long) * 2 * snap_stride(c) * (size_t)c->cap, s));
-        CUDA_TRY(cudaMemsetAsync(g->d_tpres, 0, sizeof(unsigned long long) * 4 * (size_t)c->cap, s));
-    }
+    CUDA_TRY(cudaMemsetAsync(g->d_tsnap, 0, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap, s));
+    CUDA_TRY(cudaMemsetAsync(g->d_tpres, 0, sizeof(unsigned long long) * 4 * (size_t)c->cap, s));
     // event nodes bracketing the launch: the elapsed time of the latest
     // replay is the kernel's duration on this stream
     CUDA_TRY(cudaEventRecordWithFlags(g->ev_ps[0], s, cudaEventRecordExternal));
@@ -530,7 +528,6 @@ void graph_release(amr_ctx* c) {
     if (g->d_pres3) cudaFree(g->d_pres3);
     if (g->d_pnest) cudaFree(g->d_pnest);
     if (g->d_bar) cudaFree(g->d_bar);
-    if (g->d_rpub) cudaFree(g->d_rpub);
     if (g->d_tsnap) cudaFree(g->d_tsnap);
     if (g->d_tpres) cudaFree(g->d_tpres);
     for (cudaEvent_t e : g->ev_ps)

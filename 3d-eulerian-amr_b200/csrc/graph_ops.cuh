@@ -93,14 +93,14 @@ __device__ inline double nested_sum_smem_in(const LevelLists& L, const double* l
 // coordinates t1 (along the lower of the two other axes) and t2 (the
 // higher), 1..NX.  t1 runs fastest, so the cells a warp relaxes (x fastest)
 // write neighbouring entries of every face, and the ghost faces a warp
-// fetches (relax_ghost_cell, t1 fastest) read neighbouring entries.
+// fetches (relax_ghost, t1 fastest) read neighbouring entries.
 template <int NX>
 __device__ __forceinline__ int layer_entry(int f, int t1, int t2) {
     return (f * NX + (t2 - 1)) * NX + (t1 - 1);
 }
 
-// `self`, when given, holds the brick's own values before this pass (a
-// brick kept in shared memory); else they are read from dphi.
+// `self`, when given, is the staged brick with its values before this pass
+// (relax_at); else they are read from dphi.
 template <int NX, typename CT>
 __device__ __forceinline__ CT ghost_dphi(const Geom& g, const BrickTable& bt, const DevState& st, const CT* snap_rd,
                                          size_t stride, int b, int face, int t1, int t2,
@@ -118,30 +118,13 @@ __device__ __forceinline__ CT ghost_dphi(const Geom& g, const BrickTable& bt, co
     const int q2 = ax == 2 ? qa : t2;
     if (kind == FACE_REFLECT) {  // own value mirrored through z = 0, before this pass
         const int kk = q2 == 1 ? P - 2 : 1;
-        return self ? self[(kk * P + q1) * P + q0] : D[(size_t)b * P * P * P + (kk * P + q1) * P + q0];
+        return self ? self[relax_at<NX>(q0, q1, kk)] : D[(size_t)b * P * P * P + (kk * P + q1) * P + q0];
     }
     const int v = (face & 1) ? 1 : -1;
     const int r0 = (bt.off[3 * b + 0] + (ax == 0 ? v * (P - 2) : 0) - 2 * bt.off[3 * nbr + 0] - (g.bw - 1) + q0) / 2;
     const int r1 = (bt.off[3 * b + 1] + (ax == 1 ? v * (P - 2) : 0) - 2 * bt.off[3 * nbr + 1] - (g.bw - 1) + q1) / 2;
     const int r2 = (bt.off[3 * b + 2] + (ax == 2 ? v * (P - 2) : 0) - 2 * bt.off[3 * nbr + 2] - (g.bw - 1) + q2) / 2;
     return D[(size_t)nbr * P * P * P + (r2 * P + r1) * P + r0];
-}
-
-// Ghost face cell q (< 6 NX^2) of the (NX+2)^3 brick, and its face
-// coordinates.
-template <int NX>
-__device__ __forceinline__ int relax_ghost_cell(int q, int& face, int& t1, int& t2) {
-    constexpr int P = NX + 2, F = NX * NX;
-    face = q / F;
-    const int qq = q % F;
-    t1 = qq % NX + 1;
-    t2 = qq / NX + 1;
-    const int ax = face >> 1;
-    int d[3];
-    d[ax] = (face & 1) ? P - 1 : 0;
-    d[ax == 0 ? 1 : 0] = t1;
-    d[ax == 2 ? 1 : 2] = t2;
-    return (d[2] * P + d[1]) * P + d[0];
 }
 
 // Where interior cell t (interior index) lies on a face, writes its value to
@@ -158,26 +141,36 @@ __device__ __forceinline__ void relax_layer_put(CT* sw, int t, CT v) {
     if (ck == NX) sw[layer_entry<NX>(5, ci, cj)] = v;
 }
 
-// relax_layer_put for a snapshot of tagged entries (64 bits: the FP32 value
-// in the low half, the pass word `tag` in the high half), each written with
-// one relaxed 64-bit store: a reader that sees the tag it waits for sees
-// that pass's value, with no fence and no flag between them.
-__device__ __forceinline__ void tagged_put(unsigned long long* p, float v, unsigned tag) {
-    const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
+// A tagged word: 32 bits of a value in the low half, the pass word `tag` in
+// the high half, written with one relaxed 64-bit store: a reader that sees
+// the tag it waits for sees that pass's bits, with no fence and no flag
+// between them.
+__device__ __forceinline__ void tagged_put(unsigned long long* p, unsigned bits, unsigned tag) {
+    const unsigned long long w = ((unsigned long long)tag << 32) | bits;
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
 }
-// Only the faces in `faces` (bit f for face f) are written: a layer is read
-// only by the same-level neighbour across that face.
-template <int NX>
-__device__ __forceinline__ void relax_layer_put_tagged(unsigned long long* sw, int t, float v, unsigned tag,
+// Entry e of a layer: one word for an FP32 value, two (high half first) for
+// an FP64 one.
+__device__ __forceinline__ void tagged_put_entry(unsigned long long* sw, int e, float v, unsigned tag) {
+    tagged_put(sw + e, __float_as_uint(v), tag);
+}
+__device__ __forceinline__ void tagged_put_entry(unsigned long long* sw, int e, double v, unsigned tag) {
+    tagged_put(sw + 2 * e, (unsigned)__double2hiint(v), tag);
+    tagged_put(sw + 2 * e + 1, (unsigned)__double2loint(v), tag);
+}
+// relax_layer_put for a snapshot of tagged entries.  Only the faces in
+// `faces` (bit f for face f) are written: a layer is read only by the
+// same-level neighbour across that face.
+template <int NX, typename CT>
+__device__ __forceinline__ void relax_layer_put_tagged(unsigned long long* sw, int t, CT v, unsigned tag,
                                                        unsigned faces) {
     const int ci = t % NX + 1, cj = (t / NX) % NX + 1, ck = t / (NX * NX) + 1;
-    if ((faces & 1u) && ci == 1) tagged_put(sw + layer_entry<NX>(0, cj, ck), v, tag);
-    if ((faces & 2u) && ci == NX) tagged_put(sw + layer_entry<NX>(1, cj, ck), v, tag);
-    if ((faces & 4u) && cj == 1) tagged_put(sw + layer_entry<NX>(2, ci, ck), v, tag);
-    if ((faces & 8u) && cj == NX) tagged_put(sw + layer_entry<NX>(3, ci, ck), v, tag);
-    if ((faces & 16u) && ck == 1) tagged_put(sw + layer_entry<NX>(4, ci, cj), v, tag);
-    if ((faces & 32u) && ck == NX) tagged_put(sw + layer_entry<NX>(5, ci, cj), v, tag);
+    if ((faces & 1u) && ci == 1) tagged_put_entry(sw, layer_entry<NX>(0, cj, ck), v, tag);
+    if ((faces & 2u) && ci == NX) tagged_put_entry(sw, layer_entry<NX>(1, cj, ck), v, tag);
+    if ((faces & 4u) && cj == 1) tagged_put_entry(sw, layer_entry<NX>(2, ci, ck), v, tag);
+    if ((faces & 8u) && cj == NX) tagged_put_entry(sw, layer_entry<NX>(3, ci, ck), v, tag);
+    if ((faces & 16u) && ck == 1) tagged_put_entry(sw, layer_entry<NX>(4, ci, cj), v, tag);
+    if ((faces & 32u) && ck == NX) tagged_put_entry(sw, layer_entry<NX>(5, ci, cj), v, tag);
 }
 
 // Writes a relaxed interior value of cell t to dphi and to the snapshot.
@@ -200,15 +193,14 @@ __device__ __forceinline__ void op_relax_pass(const Geom& g, const BrickTable& b
     CT* D = Corr<CT>::dphi(st) + (size_t)b * P3;
     if (mode == 1) {
         for (int q = lt; q < 6 * F; q += TH) {
-            int face, t1, t2;
-            const int gi = relax_ghost_cell<NX>(q, face, t1, t2);
+            int face, t1, t2, gi, gs;
+            relax_ghost<NX>(q, face, t1, t2, gi, gs);
             D[gi] = ghost_dphi<NX, CT>(g, bt, st, snap_rd, stride, b, face, t1, t2);
         }
         sync();
     }
-    int c[K];
     CT v[K];
-    const double resid = relax_brick<NX, TH, CT>(sm, D, Corr<CT>::dphi1(st) + (size_t)b * P3, lt, c, v, sync);
+    const double resid = relax_brick<NX, TH, CT>(sm, D, Corr<CT>::dphi1(st) + (size_t)b * P3, lt, v, sync);
     CT* sw = snap_wr + (size_t)b * stride;
 #pragma unroll
     for (int r = 0; r < K; r++) relax_put<NX, CT>(D, sw, relax_index<NX, TH>(lt, r), v[r]);

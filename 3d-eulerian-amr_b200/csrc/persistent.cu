@@ -79,65 +79,29 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, unsigned& target, un
     return ok != 0;
 }
 
-// Level-sum mailbox.  The publishing block's thread 0 stores sum g, then
-// releases lsum_gen = g; readers acquire lsum_gen until it reaches g (the
-// generations of a launch are 1, 2, ...; a reader waiting for g never sees
-// g + 1, which is published only after a grid barrier the reader has not
-// reached yet).  lsum_wait is called by every thread of a block and returns
-// the sum in all of them; false when the solve aborted.
-__device__ __forceinline__ void lsum_publish(GridBarrier* bar, unsigned g, double r) {
-    __stcg(&bar->lsum_val[g & 1], r);
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&bar->lsum_gen), "r"(g) : "memory");
-}
-
-__device__ __forceinline__ bool lsum_wait(GridBarrier* bar, unsigned g, double& r, unsigned long long limit,
-                                          int* status) {
-    __shared__ double s_r;
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) {
-        int good = 1;
-        unsigned long long spins = 0;
-        for (;;) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&bar->lsum_gen) : "memory");
-            if ((int)(v - g) >= 0) break;
-            if ((spins & 63) == 63 && ld_volatile(&bar->abort)) {
-                good = 0;
-                break;
-            }
-            if (++spins > limit) {
-                give_up(bar, status);
-                good = 0;
-                break;
-            }
-            if (spins > 32) __nanosleep(20);
-        }
-        s_r = good ? __ldcg(&bar->lsum_val[g & 1]) : 0.0;
-        s_ok = good;
-    }
-    __syncthreads();
-    r = s_r;
-    return s_ok != 0;
-}
-
 // Block layout of the solve for bricks of NX^3 interior cells: TPB threads
 // per block, NX^3 / TPB cells per thread in the relaxation (every layout
 // gives the same results bit for bit).  With 8^3 bricks and 512 threads a
 // block relaxes two bricks at once (one per half) on levels with more
 // bricks than blocks, so it holds two staged bricks; the other layouts take
-// such levels brick by brick.  With 12^3 bricks the FP32 correction's launch
-// holds two bricks' buffers, so that levels of up to twice as many bricks as
-// worker blocks stay in the shared-memory relaxation loop.  MINB: blocks per
-// SM the registers are budgeted for.
+// such levels brick by brick.  MINB: blocks per SM the registers are
+// budgeted for.  resb: the bricks one block can hold in the shared-memory
+// relaxation loop, as many as leave room for MINB blocks per SM (three
+// buffers and dphi1 each: 28 KB for an 8^3 brick in FP64, 80 KB for a 12^3
+// one, half of that in FP32).  A level of more bricks than that goes through
+// the grid barrier once a pass, at 12.7 us a pass for the 408 bricks of the
+// 4-level star on 296 blocks, against 7 us for its levels held in shared
+// memory.
 template <int NX, int TPB_>
 struct SolveLayout {
     static constexpr int TPB = TPB_;
     static constexpr bool HALVES = NX == 8 && TPB == 512;
     static constexpr int NSM = HALVES ? 2 : 1;
-    // FP32 corrections of 12^3 bricks: three more brick buffers, for a
-    // second brick per block in the shared-memory relaxation loop
-    static constexpr bool RES2 = NX == 12;
-    static_assert(!RES2 || NSM == 1, "the extra buffers follow the third brick buffer");
+    template <typename CT>
+    static constexpr int resb() {
+        if (NX == 8) return TPB == 512 ? (sizeof(CT) == 4 ? 4 : 3) : (sizeof(CT) == 4 ? 2 : 1);
+        return TPB == 864 ? (sizeof(CT) == 4 ? 4 : 2) : TPB == 576 && sizeof(CT) == 4 ? 2 : 1;
+    }
     static constexpr int MINB = TPB >= 864 ? 1 : (TPB > 288 ? 2 : (TPB > 256 ? 3 : 4));
     // threads per face in the face-ghost phases
     static constexpr int PF = NX * NX <= TPB / 6 ? NX * NX : TPB / 6;
@@ -149,7 +113,6 @@ struct Solver {
     static constexpr int TPB = Lay::TPB;
     const SolveArgs& a;
     RelaxSmem<NX, CT>* sm;  // Lay::NSM staged bricks
-    CT* xbuf;               // a third brick buffer of (NX+2)^3 entries
     double* red;
     double* nbuf;    // 2 * NEST_SMEM doubles of shared memory for the level sums
     double* nest;    // this block's scratch [cap] (level sums of larger trees)
@@ -170,8 +133,7 @@ struct Solver {
     unsigned* lvl_n;              // relaxation passes per level
     unsigned long long* lvl_ns;   // block 0's time in each level's relaxation loops
     unsigned long long* rsplit;   // block 0: the resident loops' time split [4], passes, sweeps
-    unsigned mbar = 0;            // shared-memory address of the staging mbarrier (bulk copies)
-    unsigned mbar_parity = 0;     // phase parity of its next completion (the same in every thread)
+    double solo_sum = 0.0;        // the sum of a one-brick level's last pass
 
     __device__ static unsigned long long now() {
         unsigned long long t;
@@ -292,33 +254,24 @@ struct Solver {
         return r;
     }
 
-    __device__ void count_pass(int l) {
-        relax_calls++;
-        if (blockIdx.x == 0 && threadIdx.x == 0) lvl_n[l]++;
-    }
-
     // the level sum published as generation lsum_gen (block 0 records the
-    // time it waits for it)
+    // time it waits for it).  Its two tagged halves carry the generation they
+    // belong to, so a half of another sum is never taken for this one.  Two
+    // mailboxes in turn: the server can be one generation ahead of a block
+    // that has not read this one yet, never two (serve_sum).
     __device__ bool wait_sum(double& r) {
         const unsigned long long t0 = (blockIdx.x == 0 && threadIdx.x == 0) ? now() : 0;
-        bool ok;
-        if constexpr (TAGGED) {
-            // the two tagged halves: each carries the generation it belongs
-            // to, so a half of an older sum is never taken for this one
-            __shared__ double s_r;
-            __shared__ int s_ok;
-            if (threadIdx.x == 0) {
-                CT hi, lo;
-                const int good = tagged_get2(a.bar->lsum_tag, lsum_gen, hi, lo);
-                s_r = good ? join_halves(hi, lo) : 0.0;
-                s_ok = good;
-            }
-            __syncthreads();
-            r = s_r;
-            ok = s_ok != 0;
-        } else {
-            ok = lsum_wait(a.bar, lsum_gen, r, spin_limit, &a.ctl->status);
+        __shared__ double s_r;
+        __shared__ int s_ok;
+        if (threadIdx.x == 0) {
+            unsigned hi, lo;
+            const int good = tagged_get2(a.bar->lsum_tag + 2 * (lsum_gen & 1), lsum_gen, hi, lo);
+            s_r = good ? join_halves(hi, lo) : 0.0;
+            s_ok = good;
         }
+        __syncthreads();
+        r = s_r;
+        const bool ok = s_ok != 0;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             ph_wait[PH_COUNT] += now() - t0;
             ph_wait[PH_COUNT + 1]++;
@@ -345,7 +298,7 @@ struct Solver {
             if (t < 6 * PF) op_dphi_faces<CT>(a.g, a.bt, a.st, a.aux, sl[q], t / PF, t % PF, PF);
         });
         if (!sync(PH_DPHI_FACES, n)) return false;
-        if (n <= (RES2 ? 2 * ((int)gridDim.x - 1) : (int)gridDim.x)) return relax_loop_resident(l, ratio, sl, n, snap);
+        if (n <= (int)gridDim.x || n <= RESB * ((int)gridDim.x - 1)) return relax_loop_resident(l, ratio, sl, n);
         int par = 0;
         double* pres = a.pres + (size_t)relax_par * a.L.cap;
         relax_pass(sl, n, 0, snap, snap, pres);
@@ -377,100 +330,59 @@ struct Solver {
         return true;
     }
 
-    // Thread 0 of lanes: waits until the word at p reaches target (acquire);
-    // false when the solve aborted or the wait ran out.
-    __device__ bool wait_word(const unsigned* p, unsigned target) {
-        unsigned long long spins = 0;
-        for (;;) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-            if ((int)(v - target) >= 0) return true;
-            if ((spins & 63) == 63 && ld_volatile(&a.bar->abort)) return false;
-            if (++spins > spin_limit) {
-                give_up(a.bar, &a.ctl->status);
-                return false;
-            }
-            if (spins > 32) __nanosleep(20);
-        }
+    // A pass's face layers and its sum travel as tagged entries: 32 bits of
+    // the value and the pass word in one 64-bit store (tagged_put; an FP64
+    // value is two such words).  A reader waits on the very words it reads, so
+    // a pass needs neither a block barrier nor a release fence before its
+    // layers are visible, nor a flag.  The buffers are zeroed before every
+    // launch and pass words start at 1.
+    static constexpr int RESB = Lay::template resb<CT>();
+    static constexpr int WORDS = sizeof(CT) / 4;  // tagged words of a layer entry
+    __device__ unsigned long long* tagged_snap(int p, int b) const {
+        return a.tsnap + ((size_t)p * a.snap_half + (size_t)b * a.stride) * WORDS;
+    }
+    __device__ unsigned long long* tagged_sum(const double* pres, int b) const {
+        return a.tpres + ((size_t)((pres - a.pres) / a.L.cap) * a.L.cap + b) * 2;
     }
 
-    // Waits (lanes 0-5 of warp 0, one per face) until brick b's same-level
-    // neighbours have published pass `seq`; every thread then sees their
-    // snapshot layers.
-    __device__ bool wait_neighbours(int b, unsigned seq) {
-        __shared__ int s_ok;
-        if (threadIdx.x < 32) {
-            int good = 1;
-            const int f = threadIdx.x;
-            if (f < 6 && a.bt.ftype[6 * b + f] == FACE_SIB) good = wait_word(a.rpub + a.bt.fnbr[6 * b + f], seq);
-            good = __all_sync(0xffffffffu, good);
-            if (threadIdx.x == 0) s_ok = good;
-        }
-        __syncthreads();
-        return s_ok != 0;
-    }
-
-    // The FP32 correction publishes its face layers as tagged entries (each
-    // value with its pass word in one 64-bit store, tagged_put): a neighbour
-    // waits on the very values it reads, so a pass needs neither a block
-    // barrier nor a release fence before its layers are visible, nor a
-    // separate pass word.  The FP64 correction has no room for a tag in a
-    // 64-bit store and publishes through the pass words.
-    static constexpr bool TAGGED = sizeof(CT) == 4;
-    // the launch holds a second brick's three buffers after xbuf, so the
-    // shared-memory loop takes levels of up to two bricks per worker block
-    static constexpr bool RES2 = Lay::RES2 && TAGGED;
-    // snapshot buffer p of tagged entries (their own allocation, zeroed
-    // before every launch; pass words start at 1)
-    __device__ unsigned long long* tagged_snap(int p) const { return a.tsnap + (size_t)p * a.snap_half; }
-
-    // Publishes the relaxed brick `res` as a pass: its first interior layers
-    // to snapshot buffer `wpar`, its sum to pres[b] (tagged: both as tagged
-    // entries; untagged: then brick b's pass word is released as `seq`).
-    __device__ void resident_publish(int b, const CT* res, const int* c, int wpar, double* pres, double resid,
-                                     unsigned seq) {
+    // Publishes the first interior layers of the relaxed brick `res` to
+    // snapshot buffer `wpar` as pass word `seq`: those a same-level neighbour
+    // reads (the other faces' ghosts come from the parent, the mirror or the
+    // outflow value).
+    __device__ void put_layers(int b, unsigned res, int wpar, unsigned seq) {
         constexpr int K = NX * NX * NX / TPB;
-        if constexpr (TAGGED) {
-            unsigned long long* sw = tagged_snap(wpar) + (size_t)b * a.stride;
-            // the layers a same-level neighbour reads (the other faces' ghosts
-            // come from the parent, the mirror or the outflow value)
-            unsigned sib = 0;
+        unsigned long long* sw = tagged_snap(wpar, b);
+        unsigned sib = 0;
 #pragma unroll
-            for (int f = 0; f < 6; f++) sib |= a.bt.ftype[6 * b + f] == FACE_SIB ? 1u << f : 0u;
+        for (int f = 0; f < 6; f++) sib |= a.bt.ftype[6 * b + f] == FACE_SIB ? 1u << f : 0u;
 #pragma unroll
-            for (int r = 0; r < K; r++)
-                relax_layer_put_tagged<NX>(sw, relax_index<NX, TPB>(threadIdx.x, r), float(res[c[r]]), seq, sib);
-            if (threadIdx.x == 0) {
-                // the FP64 sum as two tagged halves (pres buffer of this pass)
-                const int pp = (int)((pres - a.pres) / a.L.cap);
-                unsigned long long* w = a.tpres + ((size_t)pp * a.L.cap + b) * 2;
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(resid);
-                tagged_put(w, __uint_as_float((unsigned)(bits >> 32)), seq);
-                tagged_put(w + 1, __uint_as_float((unsigned)bits), seq);
-            }
-        } else {
-            CT* sw = reinterpret_cast<CT*>(a.snap) + (size_t)wpar * a.snap_half + (size_t)b * a.stride;
-#pragma unroll
-            for (int r = 0; r < K; r++)
-                relax_layer_put<NX, CT>(sw, relax_index<NX, TPB>(threadIdx.x, r), res[c[r]]);
-            if (threadIdx.x == 0) pres[b] = resid;
-            __syncthreads();
-            if (threadIdx.x == 0)
-                asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.rpub + b), "r"(seq) : "memory");
+        for (int r = 0; r < K; r++) {
+            const int t = relax_index<NX, TPB>(threadIdx.x, r);
+            relax_layer_put_tagged<NX, CT>(sw, t, smem()[res + relax_staged<NX>(t)], seq, sib);
         }
     }
 
-    // Two adjacent tagged entries (the halves of an FP64 value): waits until
-    // both carry pass word `tag`, loading the two together in every poll.
-    __device__ bool tagged_get2(const unsigned long long* p, unsigned tag, CT& hi, CT& lo) {
+    // Publishes brick b's sum of a pass (to the tagged twin of buffer pres).
+    __device__ void put_sum(int b, const double* pres, double resid, unsigned seq) {
+        if (threadIdx.x != 0) return;
+        unsigned long long* w = tagged_sum(pres, b);
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(resid);
+        tagged_put(w, (unsigned)(bits >> 32), seq);
+        tagged_put(w + 1, (unsigned)bits, seq);
+    }
+
+    // Two adjacent tagged words (the halves of an FP64 value): waits until
+    // both carry pass word `tag`, loading the two together in every poll;
+    // false when the solve aborted or the wait ran out.
+    __device__ bool tagged_get2(const unsigned long long* p, unsigned tag, unsigned& hi, unsigned& lo) {
         unsigned long long spins = 0;
         for (;;) {
             unsigned long long w0, w1;
             asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w0) : "l"(p) : "memory");
             asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w1) : "l"(p + 1) : "memory");
             if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag) {
-                hi = CT(__uint_as_float((unsigned)w0));
-                lo = CT(__uint_as_float((unsigned)w1));
+                hi = (unsigned)w0;
+                lo = (unsigned)w1;
                 return true;
             }
             if ((spins & 63) == 63 && ld_volatile(&a.bar->abort)) return false;
@@ -482,18 +394,20 @@ struct Solver {
         }
     }
 
-    // The FP64 value whose high and low 32 bits were sent as the bit
-    // patterns of two tagged FP32 entries.
-    __device__ static double join_halves(CT hi, CT lo) {
-        const unsigned long long bits = ((unsigned long long)__float_as_uint(float(hi)) << 32) |
-                                        __float_as_uint(float(lo));
-        return __longlong_as_double((long long)bits);
+    // The FP64 value of two 32-bit halves.
+    __device__ static double join_halves(unsigned hi, unsigned lo) {
+        return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
     }
 
-    // A same-level neighbour's tagged layer value: waits until the entry
-    // carries pass word `tag`; false when the solve aborted or the wait ran
-    // out.
+    // A same-level neighbour's layer value of pass word `tag`; false when the
+    // solve aborted or the wait ran out.
     __device__ bool tagged_get(const unsigned long long* p, unsigned tag, CT& v) {
+        if constexpr (WORDS == 2) {
+            unsigned hi, lo;
+            if (!tagged_get2(p, tag, hi, lo)) return false;
+            v = CT(join_halves(hi, lo));
+            return true;
+        }
         unsigned long long spins = 0;
         for (;;) {
             unsigned long long w;
@@ -512,115 +426,47 @@ struct Solver {
     }
 
     // One pass of brick b from its committed values in `base`, ghost faces
-    // from snapshot `rd` (the parent across coarse-fine faces, the mirror of
-    // `base` across z = 0, 0 on outflow faces), swept in x and y; nothing is
-    // written outside shared memory.  Returns the sum and the buffer with the
-    // relaxed brick (x or y).
-    __device__ double resident_pass(int b, CT* base, CT* x, CT* y, int rpar, unsigned want, const int* c,
-                                    const CT* d1, CT** res, bool& ok) {
+    // from snapshot `rpar` as pass word `want` (the parent across coarse-fine
+    // faces, the mirror of `base` across z = 0, 0 on outflow faces), swept in
+    // x and y; nothing is written outside shared memory.  Returns the sum and
+    // the buffer with the relaxed brick (x or y).
+    __device__ double resident_pass(int b, unsigned base, unsigned x, unsigned y, int rpar, unsigned want,
+                                    const CT* d1, unsigned* res, bool& ok) {
         constexpr int K = NX * NX * NX / TPB, F = NX * NX;
+        unsigned long long tt = (blockIdx.x == 0 && threadIdx.x == 0) ? now() : 0;
 #pragma unroll
-        for (int r = 0; r < K; r++) x[c[r]] = base[c[r]];
-        const CT* rd = reinterpret_cast<const CT*>(a.snap) + (size_t)rpar * a.snap_half;
+        for (int r = 0; r < K; r++) {
+            const int q = relax_staged<NX>(relax_index<NX, TPB>(threadIdx.x, r));
+            smem()[x + q] = smem()[base + q];
+        }
         int bad = 0;
         for (int q = threadIdx.x; q < 6 * F; q += TPB) {
-            int face, t1, t2;
-            const int gi = relax_ghost_cell<NX>(q, face, t1, t2);
+            int face, t1, t2, cell, gi;
+            relax_ghost<NX>(q, face, t1, t2, cell, gi);
             CT v;
-            if (TAGGED && a.bt.ftype[6 * b + face] == FACE_SIB) {
+            if (a.bt.ftype[6 * b + face] == FACE_SIB) {
                 const int nbr = a.bt.fnbr[6 * b + face];
-                const unsigned long long* p =
-                    tagged_snap(rpar) + (size_t)nbr * a.stride + layer_entry<NX>(face ^ 1, t1, t2);
-                if (!tagged_get(p, want, v)) {
+                if (!tagged_get(tagged_snap(rpar, nbr) + layer_entry<NX>(face ^ 1, t1, t2) * WORDS, want, v)) {
                     bad = 1;
                     v = CT(0);
                 }
             } else {
-                v = ghost_dphi<NX, CT>(a.g, a.bt, a.st, rd, a.stride, b, face, t1, t2, base);
+                v = ghost_dphi<NX, CT>(a.g, a.bt, a.st, nullptr, a.stride, b, face, t1, t2, smem() + base);
             }
-            x[gi] = v;
-            y[gi] = v;
+            smem()[x + gi] = v;
+            smem()[y + gi] = v;
         }
         ok = !__syncthreads_or(bad);
         if (!ok) return 0.0;
+        split(0, tt);
         int sw;
-        const double r = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, c, d1, res, BlockSync{}, &sw);
+        const double r = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, d1, res, BlockSync{}, &sw);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             rsplit[4]++;
             rsplit[5] += sw;
         }
+        split(1, tt);
         return r;
-    }
-
-    // Waits (every thread) until the staging mbarrier completes its current
-    // phase; false when the wait ran out (the solve is then aborted, and
-    // the wait goes on, again bounded, so that no copy is still landing in
-    // shared memory when the block leaves).
-    __device__ bool wait_staged() {
-        unsigned long long spins = 0;
-        bool ok = true;
-        for (;;) {
-            unsigned done;
-            asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                : "=r"(done)
-                : "r"(mbar), "r"(mbar_parity)
-                : "memory");
-            if (done) break;
-            if (++spins > spin_limit) {
-                if (!ok) break;
-                ok = false;
-                spins = 0;
-                if (threadIdx.x == 0) give_up(a.bar, &a.ctl->status);
-            }
-        }
-        mbar_parity ^= 1;
-        return ok;
-    }
-
-    // Brick b's (NX+2)^3 correction values from dphi into the two sweep
-    // buffers x and y: two bulk copies (the TMA engine, from this GPU's own
-    // memory, no multicast) issued by one thread and completed on the
-    // staging mbarrier, so the other threads load their dphi1 meanwhile.
-    // A brick is one contiguous block of P3 values whose size is a multiple
-    // of 16 bytes; where an address is not 16-byte aligned (never for the
-    // slot pool and the shared buffers, but checked) plain loads stage it.
-    // Returns whether bulk copies were issued (then wait_staged follows).
-    __device__ bool stage_brick(const CT* D, CT* x, CT* y) {
-        constexpr int P3 = (NX + 2) * (NX + 2) * (NX + 2);
-        constexpr unsigned BYTES = P3 * sizeof(CT);
-        static_assert(BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
-        const bool aligned = ((reinterpret_cast<size_t>(D) | reinterpret_cast<size_t>(x) |
-                               reinterpret_cast<size_t>(y)) & 15) == 0;
-        if (!aligned) {
-            for (int q = threadIdx.x; q < P3; q += TPB) {
-                const CT v = D[q];
-                x[q] = v;
-                y[q] = v;
-            }
-            return false;
-        }
-        // the buffers' last generic uses are over before the copies start
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const unsigned xs = (unsigned)__cvta_generic_to_shared(x);
-            const unsigned ys = (unsigned)__cvta_generic_to_shared(y);
-            // order this block's generic accesses (and, through the grid
-            // barrier before, the other blocks' writes of dphi) before the
-            // copies of the async proxy
-            asm volatile("fence.proxy.async;" ::: "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(2 * BYTES)
-                         : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(xs),
-                "l"(D), "r"(BYTES), "r"(mbar)
-                : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(ys),
-                "l"(D), "r"(BYTES), "r"(mbar)
-                : "memory");
-        }
-        return true;
     }
 
     // block 0, thread 0: adds the time since *t to split s and restarts *t
@@ -632,260 +478,230 @@ struct Solver {
         }
     }
 
-    // The server's part of a pass: waits until every brick of the level has
-    // published pass word `tag`, forms the level sum of `done` (that pass's
-    // sums) and publishes it as generation lsum_gen.  The wait is per brick:
-    // pass 1 goes out before the sum of pass 0 is known, so a count of the
-    // level's publications could be complete for pass 0 while a slow
-    // brick's pass 0 is still missing and a fast one's pass 1 is in.
+    // The server's part of a pass: takes the bricks' tagged sums of pass word
+    // `tag` straight into the shared buffer of the nested sum (or, for a level
+    // too large for it, back whole to the pres buffer `done` that the level
+    // sum reads), forms the level sum and publishes it as generation lsum_gen.
+    // A brick sends its sum of pass k + 1 before it knows the decision on pass
+    // k, so the next sum can be formed, and published in the other mailbox,
+    // while a slow block still has this one to read; the sum after that needs
+    // that block's pass k + 2, which it starts only after it has read this one.
     __device__ bool serve_sum(int l, const double* done, unsigned tag) {
-        if constexpr (TAGGED) {
-            // the bricks' tagged sums of this pass: wait on each and take it
-            // straight into the shared buffer of the nested sum (or, for a
-            // level too large for it, write it back whole to the pres
-            // buffer the level sum reads); the sum goes out as two tagged
-            // halves, so neither side needs a fence or a flag
-            const int* sl = level(l);
-            const int n = a.L.cnt[l];
-            const int pp = (int)((done - a.pres) / a.L.cap);
-            const bool in_smem = a.L.max_cnt <= NEST_SMEM;
-            int bad = 0;
-            for (int q = threadIdx.x; q < n; q += TPB) {
-                const int b = sl[q];
-                const unsigned long long* w = a.tpres + ((size_t)pp * a.L.cap + b) * 2;
-                CT hi, lo;
-                if (!tagged_get2(w, tag, hi, lo)) {
-                    bad = 1;
-                    continue;
-                }
-                if (in_smem)
-                    nbuf[q] = join_halves(hi, lo);
-                else
-                    const_cast<double*>(done)[b] = join_halves(hi, lo);
+        const int* sl = level(l);
+        const int n = a.L.cnt[l];
+        const bool in_smem = a.L.max_cnt <= NEST_SMEM;
+        int bad = 0;
+        for (int q = threadIdx.x; q < n; q += TPB) {
+            const int b = sl[q];
+            unsigned hi, lo;
+            if (!tagged_get2(tagged_sum(done, b), tag, hi, lo)) {
+                bad = 1;
+                continue;
             }
-            if (__syncthreads_or(bad)) return false;
-            const double r = !in_smem ? level_sum(l, done) : l == 0 ? nbuf[0] : nested_sum_smem_in(a.L, done, l, false, nbuf);
-            if (threadIdx.x == 0) {
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(r);
-                tagged_put(&a.bar->lsum_tag[0], __uint_as_float((unsigned)(bits >> 32)), lsum_gen);
-                tagged_put(&a.bar->lsum_tag[1], __uint_as_float((unsigned)bits), lsum_gen);
-            }
-            // the shared buffer is read again by the next pass's sum
-            __syncthreads();
-            return true;
-        } else {
-            // the bricks' pass words (a brick one pass further has put that
-            // pass's sum in the other buffer, so `done` is intact)
-            const int* sl = level(l);
-            const int n = a.L.cnt[l];
-            int bad = 0;
-            for (int q = threadIdx.x; q < n; q += TPB)
-                if (!wait_word(a.rpub + sl[q], tag)) bad = 1;
-            if (__syncthreads_or(bad)) return false;
-            const double r = level_sum(l, done);
-            if (threadIdx.x == 0) lsum_publish(a.bar, lsum_gen, r);
-            return true;
+            if (in_smem)
+                nbuf[q] = join_halves(hi, lo);
+            else
+                const_cast<double*>(done)[b] = join_halves(hi, lo);
+        }
+        if (__syncthreads_or(bad)) return false;
+        const double r = !in_smem ? level_sum(l, done) : l == 0 ? nbuf[0] : nested_sum_smem_in(a.L, done, l, false, nbuf);
+        if (threadIdx.x == 0) {
+            unsigned long long* w = a.bar->lsum_tag + 2 * (lsum_gen & 1);
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(r);
+            tagged_put(w, (unsigned)(bits >> 32), lsum_gen);
+            tagged_put(w + 1, (unsigned)bits, lsum_gen);
+        }
+        // the shared buffer is read again by the next pass's sum
+        __syncthreads();
+        return true;
+    }
+
+    // Entries, in the dynamic shared memory, of brick buffer i (0..2) of the
+    // shared-memory loop's brick j (0..RESB-1) -- the staged bricks' buffers
+    // first, then those behind them -- and of dphi1 of this thread's cells.
+    static constexpr int B3 = RelaxSmem<NX, CT>::B3;
+    static constexpr unsigned EXT = Lay::NSM * sizeof(RelaxSmem<NX, CT>) / sizeof(CT);
+    __device__ static CT* smem() { return reinterpret_cast<CT*>(dyn_smem()); }
+    __device__ static unsigned resident_buf(int j, int i) {
+        constexpr unsigned SM = sizeof(RelaxSmem<NX, CT>) / sizeof(CT);
+        const unsigned q = 3 * j + i;
+        return q < 2 * Lay::NSM ? (q / 2) * SM + (q % 2) * B3 : EXT + (q - 2 * Lay::NSM) * B3;
+    }
+    __device__ static unsigned resident_d1(int j) {
+        return EXT + (3 * RESB - 2 * Lay::NSM) * B3 + j * NX * NX * NX + threadIdx.x;
+    }
+
+    // Pass 0 of brick j in slot b: the ghost faces are in dphi (filled by the
+    // face phase).  Returns its sum, the buffer number of the result in *ri.
+    __device__ double first_pass(int j, int b, int* ri) {
+        constexpr int K = NX * NX * NX / TPB, P3 = (NX + 2) * (NX + 2) * (NX + 2);
+        const unsigned x = resident_buf(j, 0), y = resident_buf(j, 1);
+        relax_stage<NX, TPB, CT>(x, y, Corr<CT>::dphi(a.st) + (size_t)b * P3, threadIdx.x);
+        CT d1[K];
+        relax_load_d1<NX, TPB, CT>(threadIdx.x, Corr<CT>::dphi1(a.st) + (size_t)b * P3, d1);
+#pragma unroll
+        for (int r = 0; r < K; r++) smem()[resident_d1(j) + r * TPB] = d1[r];
+        __syncthreads();
+        unsigned res;
+        const double rs = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, d1, &res, BlockSync{});
+        *ri = res == x ? 0 : 1;
+        return rs;
+    }
+
+    // A later pass of brick j from its committed buffer i.
+    __device__ double next_pass(int j, int b, int i, int rpar, unsigned want, int* ri, bool& ok) {
+        constexpr int K = NX * NX * NX / TPB;
+        CT d1[K];
+#pragma unroll
+        for (int r = 0; r < K; r++) d1[r] = smem()[resident_d1(j) + r * TPB];
+        const unsigned x = resident_buf(j, (i + 1) % 3);
+        unsigned res;
+        const double rs = resident_pass(b, resident_buf(j, i), x, resident_buf(j, (i + 2) % 3), rpar, want, d1, &res,
+                                        ok);
+        *ri = res == x ? (i + 1) % 3 : (i + 2) % 3;
+        return rs;
+    }
+
+    // A committed brick back to dphi: interior and ghost faces.
+    __device__ void write_back(int b, unsigned B) {
+        constexpr int K = NX * NX * NX / TPB, P3 = (NX + 2) * (NX + 2) * (NX + 2), F = NX * NX;
+        CT* D = Corr<CT>::dphi(a.st) + (size_t)b * P3;
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+            const int t = relax_index<NX, TPB>(threadIdx.x, r);
+            D[relax_cell<NX>(t)] = smem()[B + relax_staged<NX>(t)];
+        }
+        for (int q = threadIdx.x; q < 6 * F; q += TPB) {
+            int face, t1, t2, cell, gi;
+            relax_ghost<NX>(q, face, t1, t2, cell, gi);
+            D[cell] = smem()[B + gi];
         }
     }
 
-    // Brick buffer i (0..2) of the shared-memory loop's brick j (0, 1).
-    __device__ CT* resident_buf(int j, int i) const {
-        constexpr int P3 = (NX + 2) * (NX + 2) * (NX + 2);
-        if (RES2 && j) return xbuf + (size_t)(1 + i) * P3;
-        return i == 0 ? sm[0].buf[0] : i == 1 ? sm[0].buf[1] : xbuf;
+    // what every block keeps of a finished loop whose last published pass is k
+    __device__ void loop_done(unsigned k) {
+        relax_par ^= (1 + k) & 1;
+        lsum_gen += 1 + k;
+        relax_calls += k + 1;
+        // one word more than the passes published: a sum of the pass that was
+        // dropped may be out under it
+        pass_seq += k + 2;
     }
 
     // The relaxation loop of a level the blocks can hold in shared memory:
     // one brick per block, the last block (the server) forming the level
-    // sums; or, where the level has more bricks than blocks and the launch
-    // holds a second set of brick buffers (RES2), two bricks in the first
-    // worker blocks and none in the server.  The bricks stay in shared
-    // memory for the whole loop.  No grid barrier between passes: a brick
-    // waits only for its same-level neighbours' published face layers,
-    // computes the next pass from shared memory while the server forms the
-    // last pass's nested sum, and publishes it (snapshot layers, sum, pass
-    // word) once the sum says the loop goes on -- else the pass is dropped.
-    // A block with two bricks takes them one after the other in every pass;
-    // a server with a brick (as many bricks as blocks) forms the sum first,
-    // then its pass, so its brick trails the others by the sum's latency --
-    // a smaller delay than a second brick in one block.  The loop ends with
-    // one write of each brick (interior and ghost faces) back to dphi and
-    // one grid barrier.  Passes written, their values, the sums and every
-    // loop decision are those of the loop in relax_until.
-    __device__ bool relax_loop_resident(int l, double ratio, const int* sl, int n, CT* snap) {
-        constexpr int NB = RES2 ? 2 : 1;
-        constexpr int K = NX * NX * NX / TPB, P3 = (NX + 2) * (NX + 2) * (NX + 2), F = NX * NX;
+    // sums; or, where the level has more bricks than blocks, up to RESB
+    // bricks in every worker block and none in the server.  The bricks stay
+    // in shared memory for the whole loop.  No grid barrier between passes: a
+    // brick waits only for its same-level neighbours' published face layers,
+    // computes the next pass from shared memory and sends its sum, while the
+    // server forms the last pass's nested sum; that sum decides whether the
+    // pass's layers are published, else it is dropped.  A sum goes out as
+    // soon as it is known, before the decision on the pass before it, so the
+    // decision is there when the next pass is done (the wait for it was 1.7
+    // of 7.8 us a pass on the 5-level binary).  A block with several bricks
+    // takes them one after the other in every pass; a server with a brick (as
+    // many bricks as blocks) forms the sum first, then its pass, so its brick
+    // trails the others by the sum's latency -- a smaller delay than a second
+    // brick in one block.  A level of one brick (the root) needs no other
+    // block: its block decides by itself.  The loop ends with one write of
+    // each brick (interior and ghost faces) back to dphi and one grid
+    // barrier.  Passes written, their values, the sums and every loop
+    // decision are those of the loop in relax_until.
+    __device__ bool relax_loop_resident(int l, double ratio, const int* sl, int n) {
         const int W = (int)gridDim.x - 1;
-        const bool server = (int)blockIdx.x == W;
-        // this block's bricks: slot blockIdx.x (the server's too when the
-        // level has as many bricks as blocks), and slot blockIdx.x + W in
-        // the worker blocks when it has more (-1: none)
-        const bool two = n > (int)gridDim.x;
-        const int b0 = (int)blockIdx.x < n && !(two && server) ? sl[blockIdx.x] : -1;
-        const int b1 = RES2 && two && !server && (int)blockIdx.x + W < n ? sl[blockIdx.x + W] : -1;
-        const bool mine = b0 >= 0;
-        // three buffers per brick (resident_buf): its committed values (ib0,
-        // ib1) and two to sweep in.  The brick loops below are not unrolled;
-        // a brick's values are picked by selects so they stay in registers.
-        int ib0 = 0, ib1 = 0;
-        int c[K];
-        CT d1a[K], d1b[K];
+        const bool solo = n == 1;
+        const bool server = !solo && (int)blockIdx.x == W;
+        const bool many = n > (int)gridDim.x;
+        // this block's bricks are sl[blockIdx.x + j W], j < nb
+        const int nb = (int)blockIdx.x >= n || (many && server) ? 0 : many ? (n - (int)blockIdx.x + W - 1) / W : 1;
         const unsigned seq0 = pass_seq + 1;  // pass word of pass 0
-        if (!mine && !server) {
+        if (!nb && !server) {
             // a block without a brick has no part in the loop: it goes to
             // the closing barrier (one polled word instead of the loop's
-            // published sums) and takes the loop's length from the server,
-            // which stores it before it arrives there
+            // published sums) and takes the loop's length from the block
+            // that stores it before it arrives there
             if (!sync(PH_RELAX, 0)) return false;
-            const unsigned k = *(volatile const unsigned*)&a.bar->relax_done_k;
-            relax_par ^= (1 + k) & 1;
-            lsum_gen += 1 + k;
-            relax_calls += k + 1;
-            pass_seq = seq0 + k;
+            loop_done(*(volatile const unsigned*)&a.bar->relax_done_k);
             return true;
         }
-        double* pres = a.pres + (size_t)relax_par * a.L.cap;
-#pragma unroll 1
-        for (int j = 0; j < NB; j++) {
-            const int b = j ? b1 : b0;
-            if (b < 0) continue;
-            // pass 0: the ghost faces are in dphi (filled by the face phase);
-            // the brick is staged by bulk copies while dphi1 is loaded
-            const CT* D = Corr<CT>::dphi(a.st) + (size_t)b * P3;
-            CT* x = resident_buf(j, 0);
-            CT* y = resident_buf(j, 1);
-            const bool bulk = stage_brick(D, x, y);
-            CT d1[K];
-            relax_cells<NX, TPB, CT>(threadIdx.x, Corr<CT>::dphi1(a.st) + (size_t)b * P3, c, d1);
-#pragma unroll
-            for (int r = 0; r < K; r++) {
-                if (j) d1b[r] = d1[r];
-                else d1a[r] = d1[r];
-            }
-            if (bulk && !wait_staged()) return false;
-            __syncthreads();
-            CT* res;
-            const double rs = relax_sweeps_in<NX, TPB, CT>(x, y, sm[0], threadIdx.x, c, d1, &res,
-                                                           BlockSync{});
-            const int i = res == x ? 0 : 1;
-            if (j) ib1 = i;
-            else ib0 = i;
-            resident_publish(b, res, c, 0, pres, rs, seq0);
-        }
-        count_pass(l);
-        // One pass of brick j from its committed buffer, the neighbours'
-        // layers of pass `want` in snapshot buffer `rpar`: the sum, and in
-        // *ri the buffer that holds the result.
-        auto pass = [&](int j, int rpar, unsigned want, int* ri, bool& ok) -> double {
-            const int b = j ? b1 : b0;
-            const int i = j ? ib1 : ib0;
-            CT d1[K];
-#pragma unroll
-            for (int r = 0; r < K; r++) d1[r] = j ? d1b[r] : d1a[r];
-            CT* x = resident_buf(j, (i + 1) % 3);
-            CT* res;
-            const double rs = resident_pass(b, resident_buf(j, i), x, resident_buf(j, (i + 2) % 3), rpar, want, c,
-                                            d1, &res, ok);
-            *ri = res == x ? (i + 1) % 3 : (i + 2) % 3;
-            return rs;
-        };
-        // pass 1 runs whatever the first sum; that sum is formed meanwhile
-        double r0;
-        {
-            const double* done = pres;
-            relax_par ^= 1;
-            pres = a.pres + (size_t)relax_par * a.L.cap;
-            ++lsum_gen;
-            if (server && !serve_sum(l, done, seq0)) return false;
-#pragma unroll 1
-            for (int j = 0; j < NB; j++) {
-                const int b = j ? b1 : b0;
-                if (b < 0) continue;
-                if (!TAGGED && !wait_neighbours(b, seq0)) return false;
-                bool ok;
-                int ri;
-                const double rs = pass(j, 0, seq0, &ri, ok);
-                if (!ok) return false;
-                if (j) ib1 = ri;
-                else ib0 = ri;
-                resident_publish(b, resident_buf(j, ri), c, 1, pres, rs, seq0 + 1);
-            }
-            if (!wait_sum(r0)) return false;
-            count_pass(l);
-        }
-        int par = 1;         // snapshot buffer written by the last published pass
-        unsigned k = 1;      // last published pass
+        // buffer numbers (two bits a brick) of the bricks' committed values
+        // and of the pass being computed
+        unsigned ib = 0, inext = 0;
+        unsigned k = 0;  // last published pass
         int outer = 1;
-        for (;;) {
-            const double* done = pres;
-            relax_par ^= 1;
-            pres = a.pres + (size_t)relax_par * a.L.cap;
-            ++lsum_gen;
-            if (server && !serve_sum(l, done, seq0 + k)) return false;
-            // this pass of each brick, held until the sum of the last one
-            // decides whether it is published
-            int ri0 = 0, ri1 = 0;
-            double rr0 = 0.0, rr1 = 0.0;
-            unsigned long long tt = (blockIdx.x == 0 && threadIdx.x == 0) ? now() : 0;
+        auto par = [&](unsigned pass) { return a.pres + (size_t)((relax_par ^ pass) & 1) * a.L.cap; };
+        auto step = [&](unsigned pass) -> bool {  // every brick's pass; its sum sent, its layers not yet
+            inext = 0;
 #pragma unroll 1
-            for (int j = 0; j < NB; j++) {
-                const int b = j ? b1 : b0;
-                if (b < 0) continue;
-                if (!TAGGED && !wait_neighbours(b, seq0 + k)) return false;
-                split(0, tt);
-                bool ok;
+            for (int j = 0; j < nb; j++) {
+                const int b = sl[blockIdx.x + j * W];
+                bool ok = true;
                 int ri;
-                const double rs = pass(j, par, seq0 + k, &ri, ok);
+                const double rs = pass == 0 ? first_pass(j, b, &ri)
+                                            : next_pass(j, b, (ib >> (2 * j)) & 3, (pass - 1) & 1, seq0 + pass - 1, &ri,
+                                                        ok);
                 if (!ok) return false;
-                if (j) {
-                    ri1 = ri;
-                    rr1 = rs;
-                } else {
-                    ri0 = ri;
-                    rr0 = rs;
-                }
-                split(1, tt);
+                inext |= (unsigned)ri << (2 * j);
+                if (solo)
+                    solo_sum = rs;
+                else
+                    put_sum(b, par(pass), rs, seq0 + pass);
             }
-            double r;
-            if (!wait_sum(r)) return false;
-            split(2, tt);
+            return true;
+        };
+        auto publish = [&](unsigned pass) {  // the pass just computed becomes the committed one
+            ib = inext;
+            if (!solo)
+#pragma unroll 1
+                for (int j = 0; j < nb; j++)
+                    put_layers(sl[blockIdx.x + j * W], resident_buf(j, (ib >> (2 * j)) & 3), pass & 1, seq0 + pass);
+            if (blockIdx.x == 0 && threadIdx.x == 0) lvl_n[l]++;
+        };
+        const unsigned gen0 = lsum_gen;
+        if (!step(0)) return false;
+        publish(0);
+        double r0 = solo_sum, r;
+        // pass 1 runs whatever the first sum; that sum is formed meanwhile
+        lsum_gen = gen0 + 1;
+        if (server && !serve_sum(l, par(0), seq0)) return false;
+        if (!step(1)) return false;
+        publish(1);
+        if (!solo && !wait_sum(r0)) return false;
+        k = 1;
+        for (;;) {
+            lsum_gen = gen0 + 1 + k;
+            if (solo) {
+                r = solo_sum;
+            } else {
+                if (server && !serve_sum(l, par(k), seq0 + k)) return false;
+                unsigned long long tt = 0;
+                // the next pass, held until the sum of the last one decides
+                // whether it is published
+                if (!step(k + 1)) return false;
+                if (blockIdx.x == 0 && threadIdx.x == 0) tt = now();
+                if (!wait_sum(r)) return false;
+                split(2, tt);
+            }
             bool again = r / r0 > ratio;
             if (again && outer > max_outer) {
                 again = false;
                 status = 1;
             }
             if (!again) break;
-            if (mine) {
-                ib0 = ri0;
-                resident_publish(b0, resident_buf(0, ib0), c, par ^ 1, pres, rr0, seq0 + k + 1);
-            }
-            if (b1 >= 0) {
-                ib1 = ri1;
-                resident_publish(b1, resident_buf(1, ib1), c, par ^ 1, pres, rr1, seq0 + k + 1);
-            }
+            if (solo && !step(k + 1)) return false;
+            unsigned long long tt = (blockIdx.x == 0 && threadIdx.x == 0) ? now() : 0;
+            publish(k + 1);
             split(3, tt);
-            par ^= 1;
             ++k;
-            count_pass(l);
             ++outer;
         }
 #pragma unroll 1
-        for (int j = 0; j < NB; j++) {
-            const int b = j ? b1 : b0;
-            if (b < 0) continue;
-            // the committed brick back to dphi: interior and ghost faces
-            CT* D = Corr<CT>::dphi(a.st) + (size_t)b * P3;
-            const CT* B = resident_buf(j, j ? ib1 : ib0);
-#pragma unroll
-            for (int r = 0; r < K; r++) D[c[r]] = B[c[r]];
-            for (int q = threadIdx.x; q < 6 * F; q += TPB) {
-                int face, t1, t2;
-                const int gi = relax_ghost_cell<NX>(q, face, t1, t2);
-                D[gi] = B[gi];
-            }
-        }
-        if (server && threadIdx.x == 0) a.bar->relax_done_k = k;  // the loop's length for the blocks without a brick
-        pass_seq = seq0 + k;
+        for (int j = 0; j < nb; j++) write_back(sl[blockIdx.x + j * W], resident_buf(j, (ib >> (2 * j)) & 3));
+        // the loop's length for the blocks without a brick
+        if ((server || solo) && threadIdx.x == 0) a.bar->relax_done_k = k;
+        lsum_gen = gen0;
+        loop_done(k);
         return sync(PH_RELAX, n * (k + 1));
     }
 
@@ -975,7 +791,8 @@ struct Solver {
 
 template <int NX, int TPB, typename CT>
 __global__ void __launch_bounds__(TPB, SolveLayout<NX, TPB>::MINB) k_solve_persistent(SolveArgs a) {
-    // the staged bricks live in dynamic shared memory
+    // the staged bricks live in dynamic shared memory, the further brick
+    // buffers of the shared-memory relaxation loop and its dphi1 behind them
     RelaxSmem<NX, CT>* sm = reinterpret_cast<RelaxSmem<NX, CT>*>(dyn_smem());
     __shared__ double red[16];
     __shared__ double nbuf[2 * NEST_SMEM];
@@ -983,10 +800,7 @@ __global__ void __launch_bounds__(TPB, SolveLayout<NX, TPB>::MINB) k_solve_persi
     // loop limits are read from the control block (set by the host before
     // every launch; a captured graph keeps its arguments)
     const int max_cycles = *(volatile int*)&a.ctl->max_cycles;
-    // the third brick buffer: the second half's staging buffer where the
-    // layout has one, else the dynamic shared memory after the staged brick
-    CT* xbuf = SolveLayout<NX, TPB>::NSM == 2 ? sm[1].buf[0] : reinterpret_cast<CT*>(sm + 1);
-    Solver<NX, TPB, CT> s{a, sm, xbuf, red, nbuf, a.nest + (size_t)blockIdx.x * a.L.cap, 0, 0, 0,
+    Solver<NX, TPB, CT> s{a, sm, red, nbuf, a.nest + (size_t)blockIdx.x * a.L.cap, 0, 0, 0,
                  *(volatile int*)&a.ctl->max_outer};
     __shared__ unsigned long long s_ph_ns[PH_COUNT];
     __shared__ unsigned s_ph_n[PH_COUNT];
@@ -1002,14 +816,6 @@ __global__ void __launch_bounds__(TPB, SolveLayout<NX, TPB>::MINB) k_solve_persi
     s.lvl_ns = s_lvl_ns;
     __shared__ unsigned long long s_rsplit[6];
     s.rsplit = s_rsplit;
-    // the mbarrier of the bulk brick copies: one arrival (the issuing
-    // thread's, with the bytes it expects) completes a phase
-    __shared__ __align__(8) unsigned long long s_mbar;
-    s.mbar = (unsigned)__cvta_generic_to_shared(&s_mbar);
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s.mbar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
     if (threadIdx.x < 6) s_rsplit[threadIdx.x] = 0;
     if (threadIdx.x < MAX_LEVELS) {
         s_lvl_n[threadIdx.x] = 0;
@@ -1078,9 +884,10 @@ __global__ void __launch_bounds__(TPB, SolveLayout<NX, TPB>::MINB) k_solve_persi
 template <int NX, int TPB, typename CT>
 constexpr size_t solve_smem() {
     using Lay = SolveLayout<NX, TPB>;
-    constexpr size_t P3 = (NX + 2) * (NX + 2) * (NX + 2);
-    return Lay::NSM * sizeof(RelaxSmem<NX, CT>) + (Lay::NSM == 1 ? sizeof(CT) * P3 : 0) +
-           (Lay::RES2 && sizeof(CT) == 4 ? 3 * sizeof(CT) * P3 : 0);
+    constexpr int B = Lay::template resb<CT>();
+    static_assert(3 * B >= 2 * Lay::NSM, "the staged bricks' buffers are the loop's first ones");
+    return Lay::NSM * sizeof(RelaxSmem<NX, CT>) +
+           sizeof(CT) * ((3 * B - 2 * Lay::NSM) * (size_t)RelaxSmem<NX, CT>::B3 + (size_t)B * NX * NX * NX);
 }
 
 namespace {

@@ -15,19 +15,14 @@ struct GridBarrier {
     unsigned int pad0;
     int abort;
     int pad;
-    // relaxation level sums published by one block: sum g of the launch in
-    // lsum_val[g & 1], then lsum_gen = g
-    unsigned int lsum_gen;
-    unsigned int pad1;
-    double lsum_val[2];
-    unsigned int pad2;
     // the last pass of the latest shared-memory relaxation loop (stored by
     // the block that forms its sums before the loop's closing barrier)
     unsigned int relax_done_k;
-    // the FP32 correction's level sums: the high and low halves of the FP64
-    // sum, each tagged with its generation (value and tag in one 64-bit
-    // word), on a cache line of their own
-    alignas(128) unsigned long long lsum_tag[2];
+    // the relaxation level sums published by one block: the high and low
+    // halves of sum g of the launch in words 2 (g & 1) and the next, each
+    // tagged with g (half and tag in one 64-bit word), on a cache line of
+    // their own
+    alignas(128) unsigned long long lsum_tag[4];
 };
 
 struct SolveArgs {
@@ -51,9 +46,10 @@ struct SolveArgs {
     double* pres;  // [3][cap]: two relaxation buffers, one for the L1 error
     double* nest;  // [blocks][cap] per-block nested-sum scratch
     void* snap;    // [2][cap][stride] face snapshots (CT entries)
-    unsigned* rpub;  // [cap] last pass a brick published in the shared-memory relaxation loops (zero per launch)
-    unsigned long long* tsnap;  // [2][cap][stride] tagged face snapshots of the FP32 correction (zero per launch)
-    unsigned long long* tpres;  // [2][cap][2] tagged halves of the per-brick relaxation sums (zero per launch)
+    // tagged face snapshots and halves of the per-brick relaxation sums of
+    // the shared-memory relaxation loops (zero per launch)
+    unsigned long long* tsnap;  // [2][cap][stride] entries of one (FP32) or two (FP64) words
+    unsigned long long* tpres;  // [2][cap][2]
     size_t stride;
     size_t snap_half;
     GridBarrier* bar;

@@ -113,11 +113,10 @@ __global__ void __launch_bounds__(RelaxThreads<NX>::value) k_relax(Geom g, DevSt
     const size_t base = (size_t)b * P3;
     const int t = threadIdx.x;
     CT* D = Corr<CT>::dphi(st);
-    int c[K];
     CT v[K];
-    const double resid = relax_brick<NX, TH, CT>(sm, D + base, Corr<CT>::dphi1(st) + base, t, c, v, BlockSync{});
+    const double resid = relax_brick<NX, TH, CT>(sm, D + base, Corr<CT>::dphi1(st) + base, t, v, BlockSync{});
 #pragma unroll
-    for (int r = 0; r < K; r++) D[base + c[r]] = v[r];
+    for (int r = 0; r < K; r++) D[base + relax_cell<NX>(relax_index<NX, TH>(t, r))] = v[r];
     if (t == 0) out[b] = resid;
 }
 // Poisson::store_phi / restore_phi / restore_half_phi (poisson.cpp:166-221).
