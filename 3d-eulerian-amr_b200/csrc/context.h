@@ -112,6 +112,8 @@ int zt_check(amr_ctx* c);  // reads and clears the EOS-failure word
 int rebuild_topology(amr_ctx* c);
 int alloc_slot(amr_ctx* c);
 void graph_release(amr_ctx* c);
+// the plain solve's V-cycle loop in one launch where that can be made (graph_host.cpp)
+int solve_on_device(amr_ctx* c, double tol, int max_cycles, double* l1_error, int* cycles, bool* done);
 // the staging buffer of the host copies holds at least `count` doubles
 int stage_reserve(amr_ctx* c, size_t count);
 }  // namespace amr

@@ -79,6 +79,8 @@ struct GraphState {
     GridBarrier* d_bar = nullptr;
     unsigned long long* d_tsnap = nullptr;  // [2][cap][6][nx][nx] tagged face snapshots, tsnap_words words an entry
     unsigned long long* d_tpres = nullptr;  // [2][cap][2] tagged per-brick relaxation sums
+    bool persistent_ready = false;  // the buffers below and the launch shape above are set
+    double* d_phikeep = nullptr;  // phi before a plain solve on the device (solve_on_device)
     cudaEvent_t ev_ps[2] = {nullptr, nullptr};  // around the last persistent launch
     double ps_ms_total = 0.0;                   // persistent launches of amr_graph_solve: device time, count
     long long ps_count = 0;
@@ -91,6 +93,38 @@ struct GraphState {
 };
 
 namespace {
+
+// Buffers and launch shape of the persistent solve.  A context that asks for
+// it (amr_config.persistent_solve > 0) starts with layout 0 and that many
+// blocks per SM; the plain solve's own use (solve_on_device) takes the layout
+// that the autotuner keeps on the reference's configurations: 864 threads and
+// one block per SM for 12^3 bricks, 512 threads and two for 8^3.
+int ensure_persistent(amr_ctx* c) {
+    GraphState* g = c->gs;
+    if (g->persistent_ready) return AMR_OK;
+    const bool asked = c->cfg.persistent_solve > 0;
+    g->layout = !asked && c->geom.nx == 12 ? 1 : 0;
+    g->per_sm = asked ? c->cfg.persistent_solve : c->geom.nx == 12 ? 1 : 2;
+    g->pblocks = solve_persistent_blocks(c->geom.nx, c->geom.precision, g->per_sm, g->layout);
+    if (g->pblocks <= 0) {
+        c->err = "no cooperative launch configuration for the persistent solve";
+        return AMR_ERR_CUDA;
+    }
+    g->pnest_blocks = g->pblocks;
+    if (asked)
+        for (int l = 0; l < solve_layouts(c->geom.nx); l++)
+            g->pnest_blocks = std::max(g->pnest_blocks, solve_persistent_blocks(c->geom.nx, c->geom.precision, 0, l));
+    if (!g->d_pres3) CUDA_TRY(cudaMalloc(&g->d_pres3, sizeof(double) * 3 * (size_t)c->cap));
+    if (!g->d_pnest) CUDA_TRY(cudaMalloc(&g->d_pnest, sizeof(double) * (size_t)g->pnest_blocks * c->cap));
+    if (!g->d_bar) CUDA_TRY(cudaMalloc(&g->d_bar, sizeof(GridBarrier)));
+    if (!g->d_tsnap) CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap));
+    if (!g->d_tpres) CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
+    for (cudaEvent_t& e : g->ev_ps)
+        if (asked && !e) CUDA_TRY(cudaEventCreate(&e));
+    if (!asked && !g->d_phikeep) CUDA_TRY(cudaMalloc(&g->d_phikeep, sizeof(double) * (size_t)c->cap * c->geom.pnx3));
+    g->persistent_ready = true;
+    return AMR_OK;
+}
 
 int ensure_state(amr_ctx* c) {
     if (c->gs) return AMR_OK;
@@ -108,25 +142,7 @@ int ensure_state(amr_ctx* c) {
     }
     CUDA_TRY(cudaMalloc(&g->d_counter, sizeof(unsigned int) * 4));
     CUDA_TRY(cudaMemsetAsync(g->d_counter, 0, sizeof(unsigned int) * 4, c->stream));
-    if (c->cfg.persistent_solve) {
-        g->layout = 0;
-        g->per_sm = c->cfg.persistent_solve;
-        g->pblocks = solve_persistent_blocks(c->geom.nx, c->geom.precision, g->per_sm, g->layout);
-        if (g->pblocks <= 0) {
-            c->err = "no cooperative launch configuration for the persistent solve";
-            return AMR_ERR_CUDA;
-        }
-        g->pnest_blocks = g->pblocks;
-        for (int l = 0; l < solve_layouts(c->geom.nx); l++)
-            g->pnest_blocks = std::max(g->pnest_blocks, solve_persistent_blocks(c->geom.nx, c->geom.precision, 0, l));
-        CUDA_TRY(cudaMalloc(&g->d_pres3, sizeof(double) * 3 * (size_t)c->cap));
-        CUDA_TRY(cudaMalloc(&g->d_pnest, sizeof(double) * (size_t)g->pnest_blocks * c->cap));
-        CUDA_TRY(cudaMalloc(&g->d_bar, sizeof(GridBarrier)));
-        CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap));
-        CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
-        CUDA_TRY(cudaEventCreate(&g->ev_ps[0]));
-        CUDA_TRY(cudaEventCreate(&g->ev_ps[1]));
-    }
+    if (c->cfg.persistent_solve) TRY(ensure_persistent(c));
     // side streams for capturing nested loop bodies, created outside any capture
     for (int d = 0; d < 4; d++) {
         cudaStream_t s;
@@ -288,8 +304,14 @@ int rec_vcycle(amr_ctx* c, cudaStream_t s, int depth, cudaGraphConditionalHandle
     return launched(c, __LINE__);
 }
 
+int maxslot(amr_ctx* c) {
+    int m = 0;
+    for (int sl : c->all_slots) m = std::max(m, sl + 1);
+    return m;
+}
+
 // The V-cycle loop as one persistent cooperative kernel (persistent.cu).
-int rec_persistent(amr_ctx* c, cudaStream_t s, double tol) {
+int rec_persistent(amr_ctx* c, cudaStream_t s, double tol, bool timed) {
     GraphState* g = c->gs;
     SolveArgs a{};
     a.g = c->geom;
@@ -325,13 +347,16 @@ int rec_persistent(amr_ctx* c, cudaStream_t s, double tol) {
     CUDA_TRY(cudaMemsetAsync(g->d_bar, 0, sizeof(GridBarrier), s));
     a.tsnap = g->d_tsnap;
     a.tpres = g->d_tpres;
-    CUDA_TRY(cudaMemsetAsync(g->d_tsnap, 0, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap, s));
+    // both buffers, the slots in use
+    const size_t half = sizeof(unsigned long long) * tsnap_words(c);
+    for (int p = 0; p < 2; p++)
+        CUDA_TRY(cudaMemsetAsync((char*)g->d_tsnap + p * half * c->cap, 0, half * maxslot(c), s));
     CUDA_TRY(cudaMemsetAsync(g->d_tpres, 0, sizeof(unsigned long long) * 4 * (size_t)c->cap, s));
-    // event nodes bracketing the launch: the elapsed time of the latest
-    // replay is the kernel's duration on this stream
-    CUDA_TRY(cudaEventRecordWithFlags(g->ev_ps[0], s, cudaEventRecordExternal));
+    // event nodes bracketing a captured launch: the elapsed time of the
+    // latest replay is the kernel's duration on this stream
+    if (timed) CUDA_TRY(cudaEventRecordWithFlags(g->ev_ps[0], s, cudaEventRecordExternal));
     CUDA_TRY(launch_solve_persistent(a, g->pblocks, g->layout, s));
-    CUDA_TRY(cudaEventRecordWithFlags(g->ev_ps[1], s, cudaEventRecordExternal));
+    if (timed) CUDA_TRY(cudaEventRecordWithFlags(g->ev_ps[1], s, cudaEventRecordExternal));
     g->k_vbody = 0;
     g->k_rbody = 0;
     return launched(c, __LINE__);
@@ -349,7 +374,7 @@ int rec_solve(amr_ctx* c, cudaStream_t s, double tol, int depth) {
     }
     TRY(rec_forces(c, s));
     if (c->cfg.persistent_solve) {
-        TRY(rec_persistent(c, s, tol));
+        TRY(rec_persistent(c, s, tol, true));
     } else {
         TRY(add_while(
             c, s, depth,
@@ -376,12 +401,6 @@ int rec_enforce_boundaries(amr_ctx* c, cudaStream_t s) {
     for (int l = 0; l <= c->tree.prm.max_level; l++)
         launch_ghost_fill(c->geom, c->bt, c->st, lvl(c, l), nlvl(c, l), s);
     return launched(c, __LINE__);
-}
-
-int maxslot(amr_ctx* c) {
-    int m = 0;
-    for (int sl : c->all_slots) m = std::max(m, sl + 1);
-    return m;
 }
 
 // One RK3 step of the self-gravitating driver (binary_driver.cpp:346-459 on
@@ -513,6 +532,55 @@ int need(amr_ctx* c) {
 }  // namespace
 
 namespace amr {
+// The V-cycle loop of the plain solve as one persistent launch on the
+// context's stream, with the results of the host's loop bit for bit: the host
+// loop waits for the device after every relaxation pass to read its sums
+// (23 us a pass on a 17-brick star, of which the pass itself is 6).  *done
+// stays false, with phi as it was and no error left, where the launch cannot
+// be made (no room for its buffers, no cooperative launch, loops a launch
+// must not start) or a wait in it runs out: the caller then runs its own loop.
+int solve_on_device(amr_ctx* c, double tol, int max_cycles, double* l1_error, int* cycles, bool* done) {
+    *done = false;
+    // a profiled solve is timed kernel class by kernel class; a context that
+    // runs its graph forms persistently has its launch shape for them
+    if (c->prof.on || c->cfg.persistent_solve || max_cycles < 1 || (c->geom.nx != 8 && c->geom.nx != 12)) return AMR_OK;
+    const std::string err0 = c->err;
+    auto not_here = [&]() {
+        cudaGetLastError();
+        c->err = err0;
+        return AMR_OK;
+    };
+    if (ensure_state(c) != AMR_OK || ensure_persistent(c) != AMR_OK) return not_here();
+    GraphState* g = c->gs;
+    const size_t bytes = sizeof(double) * (size_t)maxslot(c) * c->geom.pnx3;
+    CUDA_TRY(cudaMemcpyAsync(g->d_phikeep, c->st.phi, bytes, cudaMemcpyDeviceToDevice, c->stream));
+    fill_lists(c);
+    TRY(set_limits(c, max_cycles, -1));
+    const long long vb = g->k_vbody, rb = g->k_rbody;  // those of a captured graph
+    const int rc = rec_persistent(c, c->stream, tol, false);
+    g->nlevels_captured = max_level_present(c) + 1;
+    if (rc != AMR_OK) {
+        g->k_vbody = vb, g->k_rbody = rb;
+        return not_here();
+    }
+    TRY(read_ctl(c));
+    count_replay(c, 1);
+    g->k_vbody = vb, g->k_rbody = rb;
+    const int status = g->h_ctl->status;
+    if (status == 3) {
+        CUDA_TRY(cudaMemcpyAsync(c->st.phi, g->d_phikeep, bytes, cudaMemcpyDeviceToDevice, c->stream));
+        return AMR_OK;
+    }
+    *done = true;
+    *l1_error = g->h_ctl->err;
+    *cycles = g->h_ctl->cycles;
+    if (status) {
+        c->err = status == 2 ? "Poisson solve exceeded max_cycles" : "relaxation did not reach its residual ratio";
+        return AMR_ERR_NOCONVERGE;
+    }
+    return AMR_OK;
+}
+
 void graph_release(amr_ctx* c) {
     GraphState* g = c->gs;
     if (!g) return;
@@ -528,6 +596,7 @@ void graph_release(amr_ctx* c) {
     if (g->d_pres3) cudaFree(g->d_pres3);
     if (g->d_pnest) cudaFree(g->d_pnest);
     if (g->d_bar) cudaFree(g->d_bar);
+    if (g->d_phikeep) cudaFree(g->d_phikeep);
     if (g->d_tsnap) cudaFree(g->d_tsnap);
     if (g->d_tpres) cudaFree(g->d_tpres);
     for (cudaEvent_t e : g->ev_ps)

@@ -379,7 +379,15 @@ int amr_poisson_solve(amr_ctx* c, double tol, int max_cycles, double* l1_error, 
     TRY(compute_forces(c));
     double e = 0.0;
     int it = 0;
-    do {
+    bool done = false;
+    int rc = solve_on_device(c, tol, max_cycles, &e, &it, &done);
+    if (rc == AMR_OK && done) rc = check_device_error(c);
+    if (rc != AMR_OK) {
+        if (l1_error) *l1_error = e;
+        if (cycles) *cycles = it;
+        return rc;
+    }
+    if (!done) do {
         if (it >= max_cycles) {
             c->err = "Poisson solve exceeded max_cycles";
             if (l1_error) *l1_error = e;

@@ -1,9 +1,10 @@
 """The shared-memory relaxation loop of the persistent solve where it can go
 wrong: levels of one brick (decided by its own block), of as many bricks as
 blocks (the block that forms the sums holds one too), and of more (up to
-four bricks in a block), on 8^3 and 12^3 bricks, in every block layout.  The
-FP64 form must give the plain form's potential bit for bit, the mixed form
-the same bits in every layout; relaxation passes are counted alike."""
+four bricks in a block), on 8^3 and 12^3 bricks, in every block layout.  Every
+layout, and the plain solve (one launch, or the host's loop over launches
+where it is profiled), must give the same potential bit for bit in FP64 and in
+the mixed form; relaxation passes are counted alike."""
 
 import importlib.util
 import os
@@ -54,24 +55,51 @@ def test_layouts_give_the_same_bits(gpu, table_path, nx, layouts, prec):
         helm = _load_pkg_module("helm_b200", "helm.py").Helm(table_path)
         helm.set_cgs_units(P["cm"], P["g"], P["s"], 1.0)
 
-    def solve(persistent, layout=None):
+    def solve(persistent, layout=None, host_loop=True):
         a, tol = star(gpu, PREC[prec], persistent) if nx == 8 else binary(gpu, PREC[prec], persistent, helm)
         if layout is not None:
             a.set_solve_layout(*layout)
             e, n = a.graph_solve(tol)
         else:
+            a.profile(host_loop)  # a profiled solve runs the host's loop, launch by launch
             e, n = a.poisson_solve(tol)
         out = e, n, a.relax_passes(), a.download_poisson()
         a.close()
         return out
 
-    want = solve(0) if prec == "fp64" else None
+    want = solve(0)
+    got = solve(0, host_loop=False)  # the plain solve's one launch
+    assert got[:2] == want[:2] and all(np.array_equal(x, y) for x, y in zip(got[2:], want[2:]))
     for layout in layouts:
         got = solve(4, layout)
-        if want is None:
-            want = got
         assert got[0] == want[0] and got[1] == want[1], layout
         assert np.array_equal(got[2], want[2]), layout
         assert np.array_equal(got[3], want[3]), layout
     if helm is not None:
         helm.close()
+
+
+@pytest.mark.gpu
+def test_plain_solve_limits(gpu):
+    """The plain solve's one launch keeps the host loop's answers at its
+    limits: the V-cycle cap (also 0), and waits too short for the launch,
+    after which the host's loop gives the same potential."""
+    a, tol = star(gpu, 0, 0)
+    with pytest.raises(gpu.AmrError) as e:
+        a.poisson_solve(tol, 0)
+    assert e.value.code == -4
+    with pytest.raises(gpu.AmrError) as e:
+        a.poisson_solve(tol, 2)
+    assert e.value.code == -4
+    b, _ = star(gpu, 0, 0)
+    b.profile(True)
+    with pytest.raises(gpu.AmrError) as e:
+        b.poisson_solve(tol, 2)
+    assert e.value.code == -4
+    assert np.array_equal(a.download_poisson(), b.download_poisson())
+    a.set_wait_limit(1)
+    assert a.poisson_solve(tol) == b.poisson_solve(tol)
+    assert np.array_equal(a.download_poisson(), b.download_poisson())
+    a.set_wait_limit(0)
+    a.close()
+    b.close()
