@@ -20,13 +20,30 @@ template <typename T>
 __device__ __forceinline__ T r_min(T a, T b) {
     return a > b ? b : a;
 }
-template <typename T>
-__device__ __forceinline__ T r_sgn(T a) {
-    return a > T(0) ? T(1) : (a < T(0) ? T(-1) : T(0));
+// real.h:63-65: 0.5 (sgn(a) + sgn(b)) min(|a|, |b|), min(x, y) = x > y ? y : x,
+// sgn(0) = sgn(NaN) = 0.  As written that is seven FP64 operations and four
+// FP64 compares, and the two reconstructions are made of little else; the
+// same values come from one FP64 compare and the sign bits:
+//   same sign       (+-2 / 2) min = min with that sign (0 where one is 0)
+//   opposite signs  0 min: 0, or NaN for an infinite or NaN min
+//   b NaN           (sgn(a) / 2) |a|, as the comparison picks |a|
+// (A zero's sign can differ where an argument is a zero.)
+__device__ __forceinline__ bool r_isnan(double a) {
+    return (unsigned long long)__double_as_longlong(fabs(a)) > 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool r_isnan(float a) { return __float_as_uint(fabsf(a)) > 0x7f800000u; }
+__device__ __forceinline__ bool r_signs_differ(double a, double b) {
+    return (__double2hiint(a) ^ __double2hiint(b)) < 0;
+}
+__device__ __forceinline__ bool r_signs_differ(float a, float b) {
+    return (__float_as_int(a) ^ __float_as_int(b)) < 0;
 }
 template <typename T>
 __device__ __forceinline__ T minmod2(T a, T b) {
-    return T(0.5) * (r_sgn(a) + r_sgn(b)) * r_min(fabs(a), fabs(b));
+    const T fa = fabs(a), fb = fabs(b);
+    const T m = fa > fb ? fb : fa;
+    const T r = r_signs_differ(a, b) ? m - m : T(copysign(m, a));
+    return r_isnan(b) ? a * T(0.5) : r;
 }
 template <typename T>
 __device__ __forceinline__ T minmod3(T a, T b, T c) {
