@@ -174,7 +174,28 @@ int rebuild_topology(amr_ctx* c) {
         c->topo_dirty = false;
         return AMR_OK;
     }
-    // pack slot lists: all | level 0..maxl | parents 0..maxl
+    // what the one-launch ghost fill and restriction need to know of the tree
+    std::vector<int> starts;
+    c->ghost_chain = false;
+    c->h_fixes.assign(6 * (size_t)c->cap, 0);
+    auto outer_face = [&](const RefluxItem& it, int i) { return 2 * it.dir + (i == bw ? 0 : 1); };
+    for (int l = 0; l <= maxl; l++)
+        for (const RefluxItem& it : c->reflux[l])
+            if (it.i0 == bw || it.i0 == gnx - bw) c->h_fixes[6 * it.coarse + outer_face(it, it.i0)]++;
+    for (int i = 0; i < n; i++) {
+        const Node* nd = c->order[i];
+        if (nd->level > maxl) continue;
+        int refined = 0;
+        for (int ch = 0; ch < 8; ch++)
+            if (nd->child[ch] && nd->child[ch]->nchildren() > 0 && nd->child[ch]->level <= maxl) refined++;
+        c->h_refined[nd->slot] = refined;
+        if (nd->nchildren() > 0 && refined == 0) starts.push_back(nd->slot);
+        for (int f = 0; f < 6; f++)
+            if (c->h_ftype[6 * nd->slot + f] == FACE_AMR && nd->parent && ((nd->cidx >> (f >> 1)) & 1) == (f & 1) &&
+                c->h_ftype[6 * nd->parent->slot + f] == FACE_AMR)
+                c->ghost_chain = true;
+    }
+    // pack slot lists: all | level 0..maxl | parents 0..maxl | starts
     std::vector<int> packed;
     c->off_all.assign(1, 0);
     packed.insert(packed.end(), c->all_slots.begin(), c->all_slots.end());
@@ -188,6 +209,9 @@ int rebuild_topology(amr_ctx* c) {
         c->off_parent[l] = (int)packed.size();
         packed.insert(packed.end(), c->parent_slots[l].begin(), c->parent_slots[l].end());
     }
+    c->off_starts = (int)packed.size();
+    c->n_starts = (int)starts.size();
+    packed.insert(packed.end(), starts.begin(), starts.end());
     if ((int)packed.size() > c->d_slots_cap) {
         if (c->d_slots) cudaFree(c->d_slots);
         c->d_slots_cap = (int)packed.size() * 2 + 64;
@@ -211,6 +235,11 @@ int rebuild_topology(amr_ctx* c) {
     }
     c->off_reflux[maxl + 1] = (int)items.size();
     c->off_reflux_dir[3 * (maxl + 1)] = (int)items.size();
+    c->off_rstart = (int)items.size();
+    for (int l = maxl; l >= 0; l--)
+        for (const RefluxItem& it : c->reflux[l])
+            if (c->h_fixes[6 * it.child + outer_face(it, it.ic)] == 0) items.push_back(it);
+    c->n_rstart = (int)items.size() - c->off_rstart;
     // physical (non-mirror) domain faces for the multipole boundary tables
     {
         std::vector<int> bf;
@@ -350,6 +379,8 @@ int rebuild_topology(amr_ctx* c) {
     CUDA_TRY(cudaMemcpyAsync(c->bt.parent, c->h_parent.data(), sizeof(int) * m, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaMemcpyAsync(c->bt.cidx, c->h_cidx.data(), sizeof(int) * m, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaMemcpyAsync(c->bt.child, c->h_child.data(), sizeof(int) * 8 * m, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(cudaMemcpyAsync(c->d_fixes, c->h_fixes.data(), 6 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(cudaMemcpyAsync(c->d_refined, c->h_refined.data(), sizeof(int) * m, cudaMemcpyHostToDevice, c->stream));
     // host vectors may be rewritten before the async copies finish
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->topo_dirty = false;
@@ -564,7 +595,11 @@ int amr_create(const amr_config* cfg, amr_ctx** out) {
         rc |= dev_alloc(c, &c->bt.cidx, cap);
         rc |= dev_alloc(c, &c->bt.child, 8 * (size_t)cap);
         rc |= dev_alloc(c, &c->d_fo, 2 * (size_t)g.nf);
-        rc |= dev_alloc(c, &c->d_dt, cap);
+        rc |= dev_alloc(c, &c->d_dt, 3 * (size_t)cap);
+        rc |= dev_alloc(c, &c->d_refined, cap);
+        rc |= dev_alloc(c, &c->d_idone, cap);
+        rc |= dev_alloc(c, &c->d_fixes, 6 * (size_t)cap);
+        rc |= dev_alloc(c, &c->d_rdone, 6 * (size_t)cap);
         rc |= dev_alloc(c, &c->d_red, cap);
         rc |= dev_alloc(c, &c->d_flags, 8 * (size_t)cap);
         if (ztwd) {
@@ -595,6 +630,7 @@ int amr_create(const amr_config* cfg, amr_ctx** out) {
         c->h_parent.assign(cap, -1);
         c->h_cidx.assign(cap, 0);
         c->h_child.assign(8 * cap, -1);
+        c->h_refined.assign(cap, 0);
         c->free_slots.reserve(cap);
         for (int s = cap - 1; s >= 0; s--) c->free_slots.push_back(s);
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
@@ -617,6 +653,7 @@ int amr_destroy(amr_ctx* c) {
                         c->st.phi0, c->st.dphi, c->st.dphi1,  c->st.S,      c->st.fx,      c->st.fy,
                         c->st.fz,   c->bt.level, c->bt.off,   c->bt.h,      c->bt.ftype,   c->bt.fnbr,
                         c->bt.parent, c->bt.cidx, c->bt.child, c->d_fo,     c->d_dt,       c->d_red,
+                        c->d_refined, c->d_idone, c->d_fixes, c->d_rdone,
                         c->d_flags, c->d_stage, c->d_slots,  c->d_reflux, c->d_vitems, c->d_vranges, c->d_cpos,
                         c->d_U1, c->d_fwork, c->d_pubmask, c->d_pub, c->d_fdone, c->d_fctl,
                         c->st.fdphi, c->st.fdphi1, c->st.W, c->st.Vx, c->st.Vy, c->st.Vz, c->d_zerr};
@@ -771,11 +808,17 @@ int amr_synchronize(amr_ctx* c) {
     return AMR_OK;
 }
 
-// GridNode::enforce_boundaries: levels in ascending order so every
+// GridNode::enforce_boundaries: one launch where no coarse-fine ghost reads
+// another; else (and for the ZTWD state) levels in ascending order, so every
 // coarse-fine ghost reads a parent whose own ghosts are already filled.
 int amr_enforce_boundaries(amr_ctx* c) {
     NEED_DEVICE(c);
     if (is_ztwd(c)) TRY(zt_ready(c));
+    if (!is_ztwd(c) && !c->ghost_chain) {
+        ProfScope ps_(c->prof, KC_GHOST, c->stream, (long long)c->all_slots.size());
+        launch_ghost_fill_all(c->geom, c->bt, c->st, dslots_all(c), (int)c->all_slots.size(), c->stream);
+        return check_launch(c);
+    }
     for (int l = 0; l <= c->tree.prm.max_level; l++)
         {
             ProfScope ps_(c->prof, KC_GHOST, c->stream, (long long)c->level_slots[l].size());
@@ -812,8 +855,7 @@ int amr_restore(amr_ctx* c) {
     return AMR_OK;
 }
 
-// Fluxes of every brick, then coarse-fine corrections from the finest coarse
-// level upward so a corrected child face is final before its parent uses it.
+// Fluxes of every brick, then the coarse-fine corrections of every level.
 int amr_compute_fluxes(amr_ctx* c) {
     NEED_DEVICE(c);
     if (is_ztwd(c)) TRY(zt_ready(c));
@@ -825,12 +867,10 @@ int amr_compute_fluxes(amr_ctx* c) {
         else
             launch_flux(c->geom, c->st, dslots_all(c), (int)c->all_slots.size(), c->stream);
     }
-    for (int l = c->tree.prm.max_level; l >= 0; l--) {
-        const int n = c->off_reflux[l + 1] - c->off_reflux[l];
-        {
-            ProfScope ps_(c->prof, KC_REFLUX, c->stream);
-            launch_reflux(c->geom, c->st, c->d_reflux + c->off_reflux[l], n, c->stream);
-        }
+    {
+        ProfScope ps_(c->prof, KC_REFLUX, c->stream);
+        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_rstart, c->n_rstart, c->d_fixes, c->d_rdone,
+                      c->stream);
     }
     return check_launch(c);
 }
@@ -840,17 +880,14 @@ int amr_add_difs(amr_ctx* c, double dt, double beta) {
     if (is_ztwd(c)) TRY(zt_ready(c));
     const int grav = c->cfg.physics == AMR_PHYSICS_EULER_GRAVITY;
     {
-        ProfScope ps_(c->prof, KC_ADD_DIFS, c->stream);
-        launch_flow_off(c->geom, c->st, c->tree.root()->slot, c->tree.root()->h, dt, beta, c->d_fo, c->stream);
-    }
-    {
         ProfScope ps_(c->prof, KC_ADD_DIFS, c->stream, (long long)c->all_slots.size());
+        const int root = c->tree.root()->slot;
         if (is_ztwd(c))
             launch_zt_add_difs(c->geom, c->bt, c->st, c->zpar, dslots_all(c), (int)c->all_slots.size(), dt, beta,
-                               c->d_zerr, c->stream);
+                               c->d_zerr, root, c->d_fo, c->stream);
         else
-            launch_add_difs(c->geom, c->st, dslots_all(c), (int)c->all_slots.size(), c->bt.h, dt, beta, grav,
-                            c->stream);
+            launch_add_difs(c->geom, c->st, dslots_all(c), (int)c->all_slots.size(), c->bt.h, dt, beta, grav, root,
+                            c->d_fo, c->stream);
     }
     for (Node* n : c->order) n->age++;  // GridNode::add_difs, grid_node.cpp:338
     return check_launch(c);
@@ -859,53 +896,56 @@ int amr_add_difs(amr_ctx* c, double dt, double beta) {
 // Restriction from the finest parents to the root (children first).
 int amr_inject_from_children(amr_ctx* c) {
     NEED_DEVICE(c);
-    if (is_ztwd(c)) TRY(zt_ready(c));
-    for (int l = c->tree.prm.max_level; l >= 0; l--)
-        {
-            ProfScope ps_(c->prof, KC_INJECT, c->stream);
-            if (is_ztwd(c))
-                launch_zt_inject(c->geom, c->bt, c->st, c->zpar, dslots_parent(c, l), (int)c->parent_slots[l].size(),
-                                 c->d_zerr, c->stream);
-            else
-                launch_inject(c->geom, c->bt, c->st, dslots_parent(c, l), (int)c->parent_slots[l].size(),
-                              c->stream);
-        }
+    if (!is_ztwd(c)) {
+        ProfScope ps_(c->prof, KC_INJECT, c->stream);
+        launch_inject(c->geom, c->bt, c->st, c->d_slots + c->off_starts, c->n_starts, c->d_refined, c->d_idone,
+                      c->stream);
+        return check_launch(c);
+    }
+    TRY(zt_ready(c));
+    for (int l = c->tree.prm.max_level; l >= 0; l--) {
+        ProfScope ps_(c->prof, KC_INJECT, c->stream);
+        launch_zt_inject(c->geom, c->bt, c->st, c->zpar, dslots_parent(c, l), (int)c->parent_slots[l].size(),
+                         c->d_zerr, c->stream);
+    }
     return check_launch(c);
 }
 
-// Grid::max_dt per brick on the device, then GridNode::max_dt's recursion
-// (1/max of inverse child steps) on the host in the reference's order.
+// Grid::max_dt's eigenvalues per brick on the device, then GridNode::max_dt's
+// recursion (1/max of inverse child steps) on the host, children before their
+// parent; the maximum does not depend on the order of the children.
 int amr_max_dt(amr_ctx* c, double* dt) {
     NEED_DEVICE(c);
     if (!dt) return AMR_ERR_ARG;
     if (is_ztwd(c)) TRY(zt_ready(c));
     const int n = (int)c->all_slots.size();
+    int maxslot = 0;
+    for (int s : c->all_slots) maxslot = std::max(maxslot, s + 1);
     {
         ProfScope ps_(c->prof, KC_MAX_DT, c->stream, (long long)n);
         if (is_ztwd(c))
-            launch_zt_max_dt(c->geom, c->bt, c->st, c->zpar, dslots_all(c), n, c->d_dt, c->d_zerr, c->stream);
+            launch_zt_max_dt(c->geom, c->bt, c->st, c->zpar, dslots_all(c), n, c->d_dt, maxslot, c->d_zerr, c->stream);
         else
-            launch_max_dt(c->geom, c->st, dslots_all(c), n, c->bt.h, c->d_dt, c->stream);
+            launch_max_dt(c->geom, c->st, dslots_all(c), n, c->d_dt, c->stream);
     }
     TRY(check_launch(c));
     if (is_ztwd(c)) TRY(zt_check(c));
-    std::vector<double> per(c->cap);
-    int maxslot = 0;
-    for (int s : c->all_slots) maxslot = std::max(maxslot, s + 1);
-    CUDA_TRY(cudaMemcpyAsync(per.data(), c->d_dt, sizeof(double) * maxslot, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<double> lam(3 * (size_t)maxslot), dtinv(n, 0.0);
+    CUDA_TRY(cudaMemcpyAsync(lam.data(), c->d_dt, sizeof(double) * 3 * maxslot, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
-    std::function<double(const Node*)> rec = [&](const Node* nd) -> double {
-        double dtinv = 0.0;
-        for (int q = 0; q < 8; q++)
-            if (nd->child[q]) {
-                const double cdtinv = 1.0 / rec(nd->child[q]);
-                dtinv = cdtinv > dtinv ? cdtinv : dtinv;
-            }
-        const double own = 1.0 / per[nd->slot];
-        dtinv = own > dtinv ? own : dtinv;
-        return 1.0 / dtinv;
-    };
-    *dt = rec(c->tree.root());
+    for (int i = n - 1; i >= 0; i--) {  // depth-first pre-order, from its end
+        const Node* nd = c->order[i];
+        const double own = 1.0 / cfl_step(lam.data() + 3 * (size_t)nd->slot, nd->h, c->geom.cfl);
+        const double inv = own > dtinv[i] ? own : dtinv[i];
+        const double r = 1.0 / inv;
+        if (i == 0) {
+            *dt = r;
+        } else {
+            const double cdtinv = 1.0 / r;
+            double& up = dtinv[nd->parent->dfs];
+            up = cdtinv > up ? cdtinv : up;
+        }
+    }
     return AMR_OK;
 }
 

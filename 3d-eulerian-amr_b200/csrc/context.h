@@ -25,14 +25,16 @@ struct amr_ctx {
     amr::DevState st{};
     amr::BrickTable bt{};
     double* d_fo = nullptr;      // FO[nf], FO0[nf] of the root
-    double* d_dt = nullptr;      // per-slot dt / scratch [cap]
+    double* d_dt = nullptr;      // per slot: the largest eigenvalue of each direction [3 cap]
+    int* d_refined = nullptr;    // per slot: children that have children [cap]
+    unsigned* d_idone = nullptr; // per slot: of those, how many are restricted (zero between launches) [cap]
     double* d_red = nullptr;     // per-entry reduction scratch [cap]
     unsigned char* d_flags = nullptr;  // [8*cap]
     double* d_stage = nullptr;   // host<->device staging [stage_cap]
     size_t stage_cap = 0;
 
     // host mirror of the brick table
-    std::vector<int> h_level, h_off, h_ftype, h_fnbr, h_parent, h_cidx, h_child;
+    std::vector<int> h_level, h_off, h_ftype, h_fnbr, h_parent, h_cidx, h_child, h_refined;
     std::vector<double> h_h;
     std::vector<int> free_slots;
 
@@ -44,9 +46,18 @@ struct amr_ctx {
     std::vector<std::vector<amr::RefluxItem>> reflux;  // per coarse level
     int* d_slots = nullptr;                     // all_slots | level lists | parent lists
     std::vector<int> off_all, off_level, off_parent;
+    int off_starts = 0, n_starts = 0;           // in d_slots: bricks whose children are all leaves
+    // some coarse-fine ghost reads a coarse-fine ghost (never under proper nesting)
+    bool ghost_chain = false;
     amr::RefluxItem* d_reflux = nullptr;
     std::vector<int> off_reflux;
     int d_slots_cap = 0, d_reflux_cap = 0;
+    // the flux corrections' one launch: its starting items (behind the items
+    // in d_reflux), items that correct each face, counters
+    int off_rstart = 0, n_rstart = 0;
+    unsigned char* d_fixes = nullptr;  // [6 cap]
+    unsigned* d_rdone = nullptr;       // [6 cap], zero between launches
+    std::vector<unsigned char> h_fixes;
     std::vector<amr::Node*> pending_new;
     int reflux_hazards = 0;
 

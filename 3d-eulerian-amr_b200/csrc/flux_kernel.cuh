@@ -5,8 +5,14 @@
 // form's FP32 reconstruction and flux (hydro_mixed.cu) whose fluxes are
 // stored in FP64 and accumulated in FP64 by the conservative update.
 //
-// Block = one brick, 3*nx*nx threads: thread = (direction, pencil).  A pencil
-// walks its GNX cells streaming the reconstruction (recon.cuh).
+// Block = (brick, direction), three threads a pencil of nx + 1 faces; the
+// pencils' primitives are formed once a cell and staged in shared memory (37
+// KB for 8^3 bricks of bw 2, 44 KB of bw 3), and each thread streams the
+// reconstruction (recon.cuh) over its part.  The latency of FP64 divisions and
+// square roots with few warps in flight bounds it, not memory.  One thread a
+// pencil over all its cells from global memory, a block a brick, took 25.6 us
+// for 25 bricks and 69 us for 527 (minmod), 101 us for 541 (PPM), against
+// 11.8, 51.8 and 90 us now.
 #pragma once
 
 #include "recon.cuh"
@@ -23,97 +29,122 @@ __device__ __forceinline__ int flux_index(int d, int nx, int fi, int t1, int t2)
 
 __device__ __forceinline__ int cell_index(int gnx, int i, int j, int k) { return (k * gnx + j) * gnx + i; }
 
-// Primitives of cell n of one pencil (conserved state read as T, then
-// State::to_prim).
+// KT flux of one face from its reconstructed primitive states, to F (stride
+// fstride between fields).
+template <typename T, int d>
+__device__ __forceinline__ void kt_flux(T* ql, T* qr, T gam, double* F, int fstride) {
+    st_to_con(ql);
+    st_to_con(qr);
+    T fl[NF_EULER], fr[NF_EULER];
+    const T al = st_flux(ql, d, gam, fl);
+    const T ar = st_flux(qr, d, gam, fr);
+    const T a = r_max(al, ar);
+#pragma unroll
+    for (int l = 0; l < NF_EULER; l++)
+        F[l * fstride] = (double)(((fl[l] + fr[l]) - (qr[l] - ql[l]) * a) * T(0.5));
+}
+
+// Cells on each side of a face's two that its reconstruction reads, and the
+// threads of a pencil in the staged kernels.
+template <int R>
+__host__ __device__ constexpr int recon_reach() { return R == 1 ? 2 : 1; }
+constexpr int PENCIL_PARTS = 3;
+// Register budgets of the kernels: 4^3 and 8^3 bricks' blocks of at most 192
+// threads three to an SM (113 registers), 12^3 bricks' blocks of 432 one (151).
+template <bool LARGE>
+struct FluxBlock {
+    static constexpr int THREADS = PENCIL_PARTS * (LARGE ? 144 : 64), PER_SM = LARGE ? 1 : 3;
+};
+
+// Shared memory of a block, [field][cell of the pencil][pencil] with the
+// pencils padded so that staging x pencils has no bank conflicts.
+template <typename T, int R>
+inline size_t staged_smem(const Geom& g) {
+    const int npen = g.nx * g.nx, cells = g.nx + 2 * (recon_reach<R>() + 1);
+    return sizeof(T) * NF_EULER * cells * (npen + 1);
+}
+
+// Stages the primitives of every pencil cell of direction d that the faces
+// read (grid cells bw - reach - 1 ...).
+template <typename T, int d, int R>
+__device__ __forceinline__ void stage_pencils(const Geom& g, const double* Ub, T* P) {
+    const int nx = g.nx, npen = nx * nx, first = g.bw - recon_reach<R>() - 1, cells = nx + 2 * (recon_reach<R>() + 1);
+    for (int q = threadIdx.x; q < npen * cells; q += blockDim.x) {
+        // neighbouring threads on neighbouring cells in memory
+        const int n = d == 0 ? q % cells : q / npen, p = d == 0 ? q / cells : q % npen;
+        const int t1 = p % nx + g.bw, t2 = p / nx + g.bw, m = first + n;
+        const int ci = d == 0 ? cell_index(g.gnx, m, t1, t2)
+                              : (d == 1 ? cell_index(g.gnx, t1, m, t2) : cell_index(g.gnx, t1, t2, m));
+        T w[NF_EULER];
+#pragma unroll
+        for (int l = 0; l < NF_EULER; l++) w[l] = (T)Ub[l * g.gnx3 + ci];
+        st_to_prim(w);
+#pragma unroll
+        for (int l = 0; l < NF_EULER; l++) P[(l * cells + n) * (npen + 1) + p] = w[l];
+    }
+    __syncthreads();
+}
+
+// Cell n of a staged pencil; the reconstructions start as at face
+// recon_reach + 1 of a pencil whose cell 0 is the first one they read.
 template <typename T>
-struct PencilLoad {
-    const double* U;
-    int base, stride, gnx3;
+struct StagedLoad {
+    const T* P;  // cell 0 of this thread's first face
+    int row, field;
     __device__ __forceinline__ void operator()(int n, T* q) const {
 #pragma unroll
-        for (int l = 0; l < NF_EULER; l++) q[l] = (T)U[l * gnx3 + base + n * stride];
-        st_to_prim(q);
+        for (int l = 0; l < NF_EULER; l++) q[l] = P[l * field + n * row];
     }
 };
 
-// pencil p (interior transverse t1 + nx*t2) of direction d in brick b
-template <typename T, int d>
-__device__ __forceinline__ PencilLoad<T> pencil_load(const Geom& g, const double* Ub, int p) {
-    const int nx = g.nx, gnx = g.gnx, bw = g.bw;
-    const int t1 = p % nx, t2 = p / nx;
-    PencilLoad<T> L;
-    L.U = Ub;
-    L.gnx3 = g.gnx3;
-    if (d == 0) {
-        L.stride = 1;
-        L.base = cell_index(gnx, 0, t1 + bw, t2 + bw);
-    } else if (d == 1) {
-        L.stride = gnx;
-        L.base = cell_index(gnx, t1 + bw, 0, t2 + bw);
-    } else {
-        L.stride = gnx * gnx;
-        L.base = cell_index(gnx, t1 + bw, t2 + bw, 0);
+// Calls f(face 0..nx, ql, qr) for this thread's part of its pencil's faces.
+template <typename T, int R, class F>
+__device__ __forceinline__ void staged_faces(const Geom& g, const T* P, F f) {
+    const int nx = g.nx, npen = nx * nx, cells = nx + 2 * (recon_reach<R>() + 1);
+    const int p = threadIdx.x % npen, part = threadIdx.x / npen;
+    const int each = (nx + PENCIL_PARTS) / PENCIL_PARTS;
+    const int f0 = part * each, f1 = min(f0 + each, nx + 1);
+    if (f0 >= f1) return;
+    StagedLoad<T> load{P + f0 * (npen + 1) + p, npen + 1, cells * (npen + 1)};
+    constexpr int START = recon_reach<R>() + 1;  // the face f0 in load's frame
+    PencilRecon<T, R> rec;
+    rec.begin(load, START, (T)g.theta);
+    for (int q = f0; q < f1; q++) {
+        T ql[NF_EULER], qr[NF_EULER];
+        rec.next(load, START + q - f0, ql, qr);
+        f(q, ql, qr);
     }
-    return L;
 }
 
 template <typename T, int d, int R>
-__device__ __forceinline__ void flux_pencil_dir(const Geom& g, const DevState& st, int b, int p) {
-    const int nx = g.nx, gnx = g.gnx, bw = g.bw;
-    const int npen = nx * nx;
-    const int t1 = p % nx, t2 = p / nx;
-    PencilLoad<T> load = pencil_load<T, d>(g, st.U + (size_t)b * g.ucount, p);
-    double* F = (d == 0 ? st.Fx : (d == 1 ? st.Fy : st.Fz)) + (size_t)b * g.nf * npen * (nx + 1);
-    const int fstride = npen * (nx + 1);
-    const T gam = (T)g.gamma;
-    PencilRecon<T, R> rec;
-    rec.begin(load, bw, (T)g.theta);
-    for (int f = bw; f <= gnx - bw; f++) {
-        T ql[NF_EULER], qr[NF_EULER];
-        rec.next(load, f, ql, qr);
-        st_to_con(ql);
-        st_to_con(qr);
-        T fl[NF_EULER], fr[NF_EULER];
-        const T al = st_flux(ql, d, gam, fl);
-        const T ar = st_flux(qr, d, gam, fr);
-        const T a = r_max(al, ar);
-        const int fi = flux_index(d, nx, f - bw, t1, t2);
-#pragma unroll
-        for (int l = 0; l < NF_EULER; l++)
-            F[l * fstride + fi] = (double)(((fl[l] + fr[l]) - (qr[l] - ql[l]) * a) * T(0.5));
-    }
+__device__ __forceinline__ void flux_staged_dir(const Geom& g, const DevState& st, int b, T* P) {
+    const int nx = g.nx, npen = nx * nx, fstride = npen * (nx + 1);
+    stage_pencils<T, d, R>(g, st.U + (size_t)b * g.ucount, P);
+    double* F = (d == 0 ? st.Fx : (d == 1 ? st.Fy : st.Fz)) + (size_t)b * g.nf * fstride;
+    const int t1 = (threadIdx.x % npen) % nx, t2 = (threadIdx.x % npen) / nx;
+    staged_faces<T, R>(g, P, [&](int q, T* ql, T* qr) {
+        kt_flux<T, d>(ql, qr, (T)g.gamma, F + flux_index(d, nx, q, t1, t2), fstride);
+    });
 }
 
-// The direction is made a compile-time constant per thread, so the state
-// arrays indexed by it (normal velocity, normal momentum flux) stay in
-// registers.
+// grid = (bricks, 3 directions), PENCIL_PARTS nx^2 threads
 template <typename T, int R>
-__device__ __forceinline__ void flux_pencils(const Geom& g, const DevState& st, int b) {
-    const int npen = g.nx * g.nx;
-    const int d = threadIdx.x / npen;
-    const int p = threadIdx.x % npen;
-    if (d == 0)
-        flux_pencil_dir<T, 0, R>(g, st, b, p);
-    else if (d == 1)
-        flux_pencil_dir<T, 1, R>(g, st, b, p);
-    else if (d == 2)
-        flux_pencil_dir<T, 2, R>(g, st, b, p);
+__device__ __forceinline__ void flux_staged(const Geom& g, const DevState& st, int b, T* P) {
+    if (blockIdx.y == 0) flux_staged_dir<T, 0, R>(g, st, b, P);
+    else if (blockIdx.y == 1) flux_staged_dir<T, 1, R>(g, st, b, P);
+    else flux_staged_dir<T, 2, R>(g, st, b, P);
 }
 
-// Largest face eigenvalue max(lambda(ql), lambda(qr)) over the faces of
-// pencil p of direction d (Grid::max_dt's inner loop, grid.cpp:430-470).
+// Largest face eigenvalue of the staged pencils of direction d.
 template <int d, int R>
-__device__ __forceinline__ double max_eigen_pencil(const Geom& g, const DevState& st, int b, int p, double lam) {
-    PencilLoad<double> load = pencil_load<double, d>(g, st.U + (size_t)b * g.ucount, p);
-    PencilRecon<double, R> rec;
-    rec.begin(load, g.bw, g.theta);
-    for (int f = g.bw; f <= g.gnx - g.bw; f++) {
-        double ql[NF_EULER], qr[NF_EULER];
-        rec.next(load, f, ql, qr);
+__device__ __forceinline__ double max_eigen_staged(const Geom& g, const DevState& st, int b, double* P) {
+    stage_pencils<double, d, R>(g, st.U + (size_t)b * g.ucount, P);
+    double lam = 0.0;
+    staged_faces<double, R>(g, P, [&](int, double* ql, double* qr) {
         st_to_con(ql);
         st_to_con(qr);
         lam = r_max(lam, r_max(st_eigen(ql, d, g.gamma), st_eigen(qr, d, g.gamma)));
-    }
+    });
     return lam;
 }
 

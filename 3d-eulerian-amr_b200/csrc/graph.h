@@ -85,7 +85,8 @@ void launch_error_dev(const Geom& g, const BrickTable& bt, const DevState& st, c
                       double tol, cudaGraphConditionalHandle cond, Control* ctl, double* pres, double* nest,
                       unsigned int* counter, cudaStream_t s);
 void launch_open_loop(cudaGraphConditionalHandle cond, Control* ctl, int reset_cycles, cudaStream_t s);
-void launch_dt_reduce(const BrickTable& bt, const LevelLists& L, int nlevels, const double* per, double* nest,
+// lam: the eigenvalues of launch_max_dt
+void launch_dt_reduce(const BrickTable& bt, double cfl, const LevelLists& L, int nlevels, const double* lam, double* nest,
                       Control* ctl, double maxdtinc, cudaStream_t s);
 
 }  // namespace amr

@@ -390,16 +390,17 @@ int rec_solve(amr_ctx* c, cudaStream_t s, double tol, int depth) {
             launch_zt_inject(c->geom, c->bt, c->st, c->zpar, c->d_slots + c->off_parent[l],
                              (int)c->parent_slots[l].size(), c->d_zerr, s);
     } else {
-        for (int l = c->tree.prm.max_level; l >= 0; l--)
-            launch_inject(c->geom, c->bt, c->st, c->d_slots + c->off_parent[l], (int)c->parent_slots[l].size(),
-                          s);
+        launch_inject(c->geom, c->bt, c->st, c->d_slots + c->off_starts, c->n_starts, c->d_refined, c->d_idone, s);
     }
     return launched(c, __LINE__);
 }
 
 int rec_enforce_boundaries(amr_ctx* c, cudaStream_t s) {
-    for (int l = 0; l <= c->tree.prm.max_level; l++)
-        launch_ghost_fill(c->geom, c->bt, c->st, lvl(c, l), nlvl(c, l), s);
+    if (!c->ghost_chain)
+        launch_ghost_fill_all(c->geom, c->bt, c->st, all(c), nall(c), s);
+    else
+        for (int l = 0; l <= c->tree.prm.max_level; l++)
+            launch_ghost_fill(c->geom, c->bt, c->st, lvl(c, l), nlvl(c, l), s);
     return launched(c, __LINE__);
 }
 
@@ -408,8 +409,8 @@ int rec_enforce_boundaries(amr_ctx* c, cudaStream_t s) {
 int rec_step(amr_ctx* c, cudaStream_t s, double tol) {
     GraphState* g = c->gs;
     double* dtp = &g->d_ctl->dt;
-    launch_max_dt(c->geom, c->st, all(c), nall(c), c->bt.h, c->d_dt, s);
-    launch_dt_reduce(c->bt, g->L, max_level_present(c) + 1, c->d_dt, g->d_nest, g->d_ctl, c->cfg.maxdtinc, s);
+    launch_max_dt(c->geom, c->st, all(c), nall(c), c->d_dt, s);
+    launch_dt_reduce(c->bt, c->geom.cfl, g->L, max_level_present(c) + 1, c->d_dt, g->d_nest, g->d_ctl, c->cfg.maxdtinc, s);
     CUDA_TRY(cudaMemcpyAsync(c->st.U0, c->st.U, sizeof(double) * (size_t)maxslot(c) * c->geom.ucount,
                              cudaMemcpyDeviceToDevice, s));
     CUDA_TRY(cudaMemcpyAsync(c->d_fo + c->geom.nf, c->d_fo, sizeof(double) * c->geom.nf, cudaMemcpyDeviceToDevice, s));
@@ -417,12 +418,9 @@ int rec_step(amr_ctx* c, cudaStream_t s, double tol) {
     for (int rk = 0; rk < 3; rk++) {
         TRY(rec_enforce_boundaries(c, s));
         launch_flux(c->geom, c->st, all(c), nall(c), s);
-        for (int l = c->tree.prm.max_level; l >= 0; l--) {
-            const int n = c->off_reflux[l + 1] - c->off_reflux[l];
-            launch_reflux(c->geom, c->st, c->d_reflux + c->off_reflux[l], n, s);
-        }
-        launch_flow_off(c->geom, c->st, c->tree.root()->slot, c->tree.root()->h, 0.0, betas[rk], c->d_fo, s, dtp);
-        launch_add_difs(c->geom, c->st, all(c), nall(c), c->bt.h, 0.0, betas[rk], 1, s, dtp);
+        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_rstart, c->n_rstart, c->d_fixes, c->d_rdone, s);
+        launch_add_difs(c->geom, c->st, all(c), nall(c), c->bt.h, 0.0, betas[rk], 1, c->tree.root()->slot, c->d_fo, s,
+                        dtp);
         launch_phi_time(c->geom, c->st, all(c), nall(c), rk == 0 ? 0 : (rk == 1 ? 2 : 1), s);
         TRY(launched(c, __LINE__));
         TRY(rec_solve(c, s, tol, 0));

@@ -8,6 +8,7 @@
 
 #include "euler_state.cuh"
 #include "graph_ops.cuh"
+#include "kernels.h"
 #include "launch.cuh"
 
 namespace amr {
@@ -155,7 +156,7 @@ __global__ void k_open_loop(cudaGraphConditionalHandle cond, Control* ctl, int r
 // GridNode::max_dt (grid_node.cpp:163-174) over per-brick steps, then the
 // driver's MAXDTINC clamp (hydro_driver.cpp:108-113) against the previous
 // step.  One block.
-__global__ void k_dt_reduce(BrickTable bt, LevelLists L, int nlevels, const double* __restrict__ per, double* nest,
+__global__ void k_dt_reduce(BrickTable bt, double cfl, LevelLists L, int nlevels, const double* __restrict__ lam, double* nest,
                             Control* ctl, double maxdtinc) {
     // R(n) = 1 / max(1/own, max_c 1/R(c)); nest holds R
     for (int m = nlevels - 1; m >= 0; m--) {
@@ -169,7 +170,7 @@ __global__ void k_dt_reduce(BrickTable bt, LevelLists L, int nlevels, const doub
                 const double cdtinv = 1.0 / __ldcg(nest + ch);
                 dtinv = cdtinv > dtinv ? cdtinv : dtinv;
             }
-            const double own = 1.0 / __ldcg(per + p);
+            const double own = 1.0 / cfl_step(lam + 3 * (size_t)p, bt.h[p], cfl);
             dtinv = own > dtinv ? own : dtinv;
             nest[p] = 1.0 / dtinv;
         }
@@ -238,9 +239,9 @@ void launch_open_loop(cudaGraphConditionalHandle cond, Control* ctl, int reset_c
     launch_k(k_open_loop, 1, 1, 0, s, cond, ctl, reset_cycles);
 }
 
-void launch_dt_reduce(const BrickTable& bt, const LevelLists& L, int nlevels, const double* per, double* nest,
+void launch_dt_reduce(const BrickTable& bt, double cfl, const LevelLists& L, int nlevels, const double* lam, double* nest,
                       Control* ctl, double maxdtinc, cudaStream_t s) {
-    launch_k(k_dt_reduce, 1, 1024, 0, s, bt, L, nlevels, per, nest, ctl, maxdtinc);
+    launch_k(k_dt_reduce, 1, 1024, 0, s, bt, cfl, L, nlevels, lam, nest, ctl, maxdtinc);
 }
 
 }  // namespace amr

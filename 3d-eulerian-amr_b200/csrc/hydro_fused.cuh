@@ -21,111 +21,12 @@
 // so with FT = double the result is bitwise that of amr_sub_step.
 #pragma once
 
-#include "euler_state.cuh"
 #include "flux_kernel.cuh"
+#include "hydro_cell.cuh"
 #include "hydro_fused.h"
 
 namespace amr {
 
-
-// Six conserved fields of one cell, indexed only by compile-time constants
-// (stays in registers).
-struct Cell6 {
-    double v[NF_EULER];
-};
-
-// State::enforce_outflow (euler/state.cpp:45-84) on a register cell, the
-// same arithmetic as st_enforce_outflow without a run-time array index.
-__device__ __forceinline__ void fused_outflow(Cell6& u, int bface) {
-    const int m = 1 + (bface >> 1);
-    const double um = m == 1 ? u.v[1] : (m == 2 ? u.v[2] : u.v[3]);
-    bool zero;
-    if (bface == ZU || bface == ZL) {
-        zero = (bface == ZU) ? (u.v[3] > 0.0) : (u.v[3] < 0.0);
-    } else {
-        const double v = um / u.v[0];
-        zero = (bface & 1) ? (v > 0.0) : (v < 0.0);
-    }
-    if (zero) {
-        u.v[4] = u.v[4] - 0.5 * um * um / u.v[0];
-        if (m == 1) u.v[1] = 0.0;
-        else if (m == 2) u.v[2] = 0.0;
-        else u.v[3] = 0.0;
-    }
-}
-
-__device__ __forceinline__ int axis_of(int x, int y, int z, int a) { return a == 0 ? x : (a == 1 ? y : z); }
-
-__device__ __forceinline__ void fused_load(const FusedArgs& A, int b, int x, int y, int z, Cell6& u) {
-    const double* U = A.Uin + (size_t)b * A.g.ucount + cell_index(A.g.gnx, x, y, z);
-#pragma unroll
-    for (int l = 0; l < NF_EULER; l++) u.v[l] = U[(size_t)l * A.g.gnx3];
-}
-
-// Cell (x, y, z) (GNX frame) of brick b: the interior value, or the
-// face-ghost value k_ghost_fill would store there (at most one coordinate
-// outside the interior).  DEPTH bounds the coarse-fine hops: a coarse-fine
-// ghost reads the parent's cells, whose ghosts across the same face are
-// same-level or domain ghosts under proper nesting, so DEPTH = 1 suffices;
-// a deeper chain sets err bit 1.
-template <int DEPTH>
-__device__ __forceinline__ void fused_cell(const FusedArgs& A, int b, int x, int y, int z, Cell6& u) {
-    const int bw = 2, gnx = 12;
-    const int ax = (x < bw || x >= gnx - bw) ? 0 : ((y < bw || y >= gnx - bw) ? 1 : ((z < bw || z >= gnx - bw) ? 2 : -1));
-    if (ax < 0) {
-        fused_load(A, b, x, y, z, u);
-        return;
-    }
-    const int gi = axis_of(x, y, z, ax);
-    const int upper = gi >= gnx - bw ? 1 : 0;
-    const int face = 2 * ax + upper;
-    const int kind = A.bt.ftype[6 * b + face];
-    const int nbr = A.bt.fnbr[6 * b + face];
-    int sx = x, sy = y, sz = z, src = b;
-    int s;
-    if (kind == FACE_SIB) {
-        s = upper ? gi - (gnx - 2 * bw) : gi + (gnx - 2 * bw);
-        src = nbr;
-    } else if (kind == FACE_OUTFLOW) {
-        s = upper ? gnx - bw - 1 : bw;
-    } else if (kind == FACE_REFLECT) {
-        s = 2 * bw - 1 - gi;
-    } else {
-        s = -1;
-    }
-    if (s >= 0) {
-        if (ax == 0) sx = s;
-        else if (ax == 1) sy = s;
-        else sz = s;
-        fused_load(A, src, sx, sy, sz, u);
-        if (kind == FACE_OUTFLOW) fused_outflow(u, face ^ 1);
-        if (kind == FACE_REFLECT) u.v[3] = -u.v[3];
-        return;
-    }
-    if constexpr (DEPTH == 0) {
-        atomicOr(A.err, 2);
-#pragma unroll
-        for (int l = 0; l < NF_EULER; l++) u.v[l] = 0.0;
-    } else {
-        // GridAMRBound::operator() (grid_amr_bound.cpp:27-78)
-        const int fx = A.bt.off[3 * b + 0] - 2 * A.bt.off[3 * nbr + 0] + x;
-        const int fy = A.bt.off[3 * b + 1] - 2 * A.bt.off[3 * nbr + 1] + y;
-        const int fz = A.bt.off[3 * b + 2] - 2 * A.bt.off[3 * nbr + 2] + z;
-        const int px = fx / 2, py = fy / 2, pz = fz / 2;
-        const int par = axis_of(fx, fy, fz, ax) % 2;
-        const int dx = ax == 0, dy = ax == 1, dz = ax == 2;
-        Cell6 uc, up, um;
-        fused_cell<DEPTH - 1>(A, nbr, px, py, pz, uc);
-        fused_cell<DEPTH - 1>(A, nbr, px + dx, py + dy, pz + dz, up);
-        fused_cell<DEPTH - 1>(A, nbr, px - dx, py - dy, pz - dz, um);
-#pragma unroll
-        for (int l = 0; l < NF_EULER; l++) {
-            double m = minmod2(up.v[l] - uc.v[l], uc.v[l] - um.v[l]);
-            if (par == 1) m = -m;
-            u.v[l] = uc.v[l] - m * 0.25;
-        }
-    }
-}
 
 __device__ __forceinline__ void fused_wait(const FusedArgs& A, int child) {
     unsigned long long spins = 0;
@@ -167,17 +68,17 @@ __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, F
     for (int q = tid; q < CROSS; q += FUSED_BLOCK) {
         Cell6 u;
         if (q < 512) {
-            fused_load(A, b, q % 8 + bw, (q / 8) % 8 + bw, q / 64 + bw, u);
+            cell_load(A.Uin, A.g.ucount, gnx, A.g.gnx3, b, q % 8 + bw, (q / 8) % 8 + bw, q / 64 + bw, u);
         } else {
             const int r = q - 512, t1 = r % 8 + bw, t2 = (r / 8) % 8 + bw, depth = (r / 64) % 2, face = r / 128;
             const int ax = face >> 1;
             const int n = (face & 1) ? gnx - bw + depth : depth;
             if (ax == 0)
-                fused_cell<1>(A, b, n, t1, t2, u);
+                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, n, t1, t2, u, A.err);
             else if (ax == 1)
-                fused_cell<1>(A, b, t1, n, t2, u);
+                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, t1, n, t2, u, A.err);
             else
-                fused_cell<1>(A, b, t1, t2, n, u);
+                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, t1, t2, n, u, A.err);
         }
         FT w[NF_EULER];
 #pragma unroll

@@ -9,8 +9,12 @@
 //   Fz [slot][f][k'][j'][i'] faces k'=0..nx
 #include "euler_state.cuh"
 #include "flux_kernel.cuh"
+#include "flow_off.cuh"
+#include "hydro_cell.cuh"
 #include "kernels.h"
 #include "launch.cuh"
+
+#include <algorithm>
 
 namespace amr {
 
@@ -95,46 +99,116 @@ __global__ void k_ghost_fill(Geom g, BrickTable bt, DevState st, const int* __re
     }
 }
 
+// The same for every level in one launch: every ghost value is computed from
+// interior cells (ghost_cell), so no level waits for another.  Needs a tree
+// whose coarse-fine ghosts read no coarse-fine ghosts (proper nesting; the
+// host checks, and runs the level-ordered fill otherwise).  A launch of a
+// small level is 5 us of latency; one per level was 18 to 21% of a step.
+// grid = (bricks, 6 faces); neighbouring threads on neighbouring cells; the
+// brick's sizes at compile time (0: at run time) for the index divisions.
+template <int BW, int NX>
+__global__ void __launch_bounds__(128) k_ghost_fill_all(Geom g, BrickTable bt, DevState st,
+                                                        const int* __restrict__ slots) {
+    const int b = slots[blockIdx.x];
+    const int face = blockIdx.y;
+    const int ax = face >> 1, upper = face & 1;
+    const int bw = BW ? BW : g.bw, nx = NX ? NX : g.nx, gnx = nx + 2 * bw, gnx3 = gnx * gnx * gnx;
+    const int kind = bt.ftype[6 * b + face];
+    const int step = ax == 0 ? 1 : (ax == 1 ? gnx : gnx * gnx);
+    for (int t = threadIdx.x; t < bw * nx * nx; t += blockDim.x) {
+        const int n = ax == 0 ? t % bw : (t / nx) % bw;
+        const int t1 = (ax == 0 ? (t / bw) % nx : t % nx) + bw;
+        const int t2 = t / (bw * nx) + bw;
+        const int gi = upper ? gnx - bw + n : n;
+        const int x = ax == 0 ? gi : t1, y = ax == 1 ? gi : (ax == 0 ? t1 : t2), z = ax == 2 ? gi : t2;
+        const int to = cell_index(gnx, x, y, z);
+        Cell6 u;
+        if (kind == FACE_SIB) {
+            const double* V = st.U + (size_t)bt.fnbr[6 * b + face] * g.ucount + to + (upper ? -nx : nx) * step;
+#pragma unroll
+            for (int l = 0; l < NF_EULER; l++) u.v[l] = V[l * gnx3];
+        } else {
+            ghost_cell<1, BW, NX ? NX + 2 * BW : 0>(g, bt, st.U, b, x, y, z, u, nullptr);
+        }
+        double* U = st.U + (size_t)b * g.ucount + to;
+#pragma unroll
+        for (int l = 0; l < NF_EULER; l++) U[l * gnx3] = u.v[l];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // KT/Rusanov fluxes, Grid::compute_{x,y,z}_flux (grid.cpp:215-302) with
 // minmod-theta (reconstruct.cpp:60-71) or PPM (reconstruct.cpp:22-58)
-// reconstruction.  Block = one brick, 3*nx*nx threads: thread = (direction,
-// pencil).  A pencil walks its GNX cells streaming the reconstruction.
+// reconstruction (flux_kernel.cuh).  grid = (bricks, 3 directions)
 // ---------------------------------------------------------------------------
-template <int R>
-__global__ void k_flux(Geom g, DevState st, const int* __restrict__ slots) {
-    flux_pencils<double, R>(g, st, slots[blockIdx.x]);
+template <int R, bool LARGE>
+__global__ void __launch_bounds__(FluxBlock<LARGE>::THREADS, FluxBlock<LARGE>::PER_SM) k_flux(Geom g, DevState st, const int* __restrict__ slots) {
+    extern __shared__ double flux_smem[];
+    flux_staged<double, R>(g, st, slots[blockIdx.x], flux_smem);
 }
 
 // ---------------------------------------------------------------------------
 // Coarse-fine flux correction, GridNode::adjust_{x,y,z}_flux
 // (grid_node.cpp:1076-1274): the coarse face quadrant takes the mean of the
-// child's four faces.  One block per item, thread per (field, face cell).
-// Items of one coarse level run after every finer level is final.
+// child's four faces.  A child's face can itself be corrected (at a domain
+// face, where no neighbour decides: elsewhere proper nesting leaves none), so
+// the finest coarse level comes first.  One launch for all levels: a block
+// starts at an item whose child's face is not corrected and, if it is the
+// last of the items that correct the coarse brick's face, goes on to the item
+// that reads that face (a counter per brick face, back to zero for the next
+// launch); no block waits.  fixes[6 slot + face] = items that correct the
+// face.  One block per starting item, thread per (field, face cell).
 // ---------------------------------------------------------------------------
-__global__ void k_reflux(Geom g, DevState st, const RefluxItem* __restrict__ items) {
-    const RefluxItem it = items[blockIdx.x];
+__global__ void k_reflux(Geom g, BrickTable bt, DevState st, const RefluxItem* __restrict__ items,
+                         const unsigned char* __restrict__ fixes, unsigned* done) {
+    __shared__ int s_go;
+    RefluxItem it = items[blockIdx.x];
     const int nx = g.nx, bw = g.bw, gnx = g.gnx;
-    const int half = nx / 2;
+    const int half = nx / 2, fstride = nx * nx * (nx + 1);
     const int t = threadIdx.x;
-    if (t >= g.nf * half * half) return;
     const int l = t / (half * half);
     const int q = t % (half * half);
     const int a = q % half, c = q / half;      // by2 indexer: j = bw+2a, k = bw+2c
     const int j = 2 * a, k = 2 * c;            // child interior offsets
-    const int j0 = a + it.cj * half, k0 = c + it.ck * half;  // coarse interior offsets
-    const int npen = nx * nx, fstride = npen * (nx + 1);
-    double* Fbase = (it.dir == 0 ? st.Fx : (it.dir == 1 ? st.Fy : st.Fz));
-    const double* Fc = Fbase + (size_t)it.child * g.nf * fstride + l * fstride;
-    double* Fp = Fbase + (size_t)it.coarse * g.nf * fstride + l * fstride;
-    const int ic = it.ic - bw, i0 = it.i0 - bw;
-    double v = +Fc[flux_index(it.dir, nx, ic, j, k)];
-    v += Fc[flux_index(it.dir, nx, ic, j + 1, k)];
-    v += Fc[flux_index(it.dir, nx, ic, j, k + 1)];
-    v += Fc[flux_index(it.dir, nx, ic, j + 1, k + 1)];
-    v *= 0.25;
-    Fp[flux_index(it.dir, nx, i0, j0, k0)] = v;
-    (void)gnx;
+    for (;;) {
+        if (t < g.nf * half * half) {
+            const int j0 = a + it.cj * half, k0 = c + it.ck * half;  // coarse interior offsets
+            double* F = (it.dir == 0 ? st.Fx : (it.dir == 1 ? st.Fy : st.Fz));
+            const double* Fc = F + ((size_t)it.child * g.nf + l) * fstride;
+            double* Fp = F + ((size_t)it.coarse * g.nf + l) * fstride;
+            const int ic = it.ic - bw;
+            // L2 loads: another block of this launch may have corrected them,
+            // and a line of them can be in this SM's first cache already
+            double v = +__ldcg(Fc + flux_index(it.dir, nx, ic, j, k));
+            v += __ldcg(Fc + flux_index(it.dir, nx, ic, j + 1, k));
+            v += __ldcg(Fc + flux_index(it.dir, nx, ic, j, k + 1));
+            v += __ldcg(Fc + flux_index(it.dir, nx, ic, j + 1, k + 1));
+            v *= 0.25;
+            Fp[flux_index(it.dir, nx, it.i0 - bw, j0, k0)] = v;
+        }
+        // the face just corrected, if it is an outer one, and who reads it
+        if (it.i0 != bw && it.i0 != gnx - bw) return;
+        const int p = it.coarse, side = it.i0 == bw ? 0 : 1, face = 2 * it.dir + side;
+        if (bt.parent[p] < 0 || bt.ftype[6 * p + face] == FACE_SIB) return;
+        __threadfence();
+        __syncthreads();
+        if (t == 0) {
+            const bool last = atomicAdd(done + 6 * p + face, 1u) == (unsigned)fixes[6 * p + face] - 1u;
+            if (last) done[6 * p + face] = 0u;
+            s_go = last;
+        }
+        __syncthreads();
+        if (!s_go) return;
+        __threadfence();
+        const int ta = it.dir == 0 ? 1 : 0, tb = it.dir == 2 ? 1 : 2, ci = bt.cidx[p];
+        const bool outer = ((ci >> it.dir) & 1) == side;
+        it.child = p;
+        it.coarse = bt.parent[p];
+        it.ic = side ? gnx - bw : bw;
+        it.i0 = outer ? it.ic : gnx / 2;
+        it.cj = (ci >> ta) & 1;
+        it.ck = (ci >> tb) & 1;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -142,17 +216,25 @@ __global__ void k_reflux(Geom g, DevState st, const RefluxItem* __restrict__ ite
 // Grid::add_difs (grid.cpp:201-213, 304-344, 406-420).  With gravity the
 // ZSTAR energy work term and the momentum sources of the restated coupling
 // (single/single.cpp:49-97, 304-383) are added in the reference order.
-// Block = one brick, thread per interior cell.
+// grid = (bricks, cells / 256) + the root's flow-off in the last block of
+// the first row; thread per interior cell.
 // ---------------------------------------------------------------------------
-__global__ void k_add_difs(Geom g, DevState st, const int* __restrict__ slots, const double* __restrict__ hs,
-                           double dt_arg, const double* __restrict__ dtp, double beta, int gravity) {
+__global__ void __launch_bounds__(256) k_add_difs(Geom g, DevState st, const int* __restrict__ slots,
+                                                  const double* __restrict__ hs, double dt_arg,
+                                                  const double* __restrict__ dtp, double beta, int gravity, int root,
+                                                  double* fo) {
+    const double dt = dtp ? *dtp : dt_arg;  // device-computed step in captured graphs
+    if (blockIdx.x == gridDim.x - 1) {
+        if (blockIdx.y == 0) flow_off_block(g, st, root, hs[root], dt, beta, fo);
+        return;
+    }
     const int b = slots[blockIdx.x];
     const int nx = g.nx, gnx = g.gnx, bw = g.bw, pnx = g.pnx;
     const int npen = nx * nx, fstride = npen * (nx + 1);
-    const double dt = dtp ? *dtp : dt_arg;  // device-computed step in captured graphs
     const double h = hs[b];
     const double hinv = 1.0 / h;
-    for (int t = threadIdx.x; t < nx * nx * nx; t += blockDim.x) {
+    const int t = blockIdx.y * blockDim.x + threadIdx.x;
+    if (t < nx * nx * nx) {
         const int i = t % nx, j = (t / nx) % nx, k = t / npen;
         double D[NF_EULER];
 #pragma unroll
@@ -209,72 +291,75 @@ __global__ void k_add_difs(Geom g, DevState st, const int* __restrict__ slots, c
     }
 }
 
-// Root flow-off: Grid::sum_{x,y,z}_flow_off (grid.cpp:346-404) in the
-// sequential order of a one-thread OpenMP run, then FO update of
-// Grid::add_difs (grid.cpp:419).  fo = [FO(nf), FO0(nf)].  One thread/field.
-__global__ void k_flow_off(Geom g, DevState st, int root, double h, double dt_arg, const double* __restrict__ dtp,
-                           double beta, double* fo) {
-    const int l = threadIdx.x;
-    const double dt = dtp ? *dtp : dt_arg;
-    if (l >= g.nf) return;
-    const int nx = g.nx, npen = nx * nx, fstride = npen * (nx + 1);
-    const double* Fx = st.Fx + (size_t)root * g.nf * fstride + l * fstride;
-    const double* Fy = st.Fy + (size_t)root * g.nf * fstride + l * fstride;
-    const double* Fz = st.Fz + (size_t)root * g.nf * fstride + l * fstride;
-    double dfo = 0.0;
-    for (int t2 = 0; t2 < nx; t2++)
-        for (int t1 = 0; t1 < nx; t1++)
-            dfo += (Fx[flux_index(0, nx, nx, t1, t2)] - Fx[flux_index(0, nx, 0, t1, t2)]) * h * h;
-    for (int t2 = 0; t2 < nx; t2++)
-        for (int t1 = 0; t1 < nx; t1++)
-            dfo += (Fy[flux_index(1, nx, nx, t1, t2)] - Fy[flux_index(1, nx, 0, t1, t2)]) * h * h;
-    for (int t2 = 0; t2 < nx; t2++)
-        for (int t1 = 0; t1 < nx; t1++) {
-            if (g.z_reflect)
-                dfo += (Fz[flux_index(2, nx, nx, t1, t2)]) * h * h;
-            else
-                dfo += (Fz[flux_index(2, nx, nx, t1, t2)] - Fz[flux_index(2, nx, 0, t1, t2)]) * h * h;
-        }
-    fo[l] = (fo[l] + dfo * dt) * beta + fo[g.nf + l] * (1.0 - beta);
+// The root's flow-off by itself (the fused substep).
+__global__ void __launch_bounds__(256) k_flow_off(Geom g, DevState st, int root, double h, double dt, double beta,
+                                                  double* fo) {
+    flow_off_block(g, st, root, h, dt, beta, fo);
 }
 
 // ---------------------------------------------------------------------------
 // Restriction, GridNode::inject_from_children (grid_node.cpp:1035-1074):
 // covered parent cell := mean of its 8 child cells, then floor.
-// grid = (parents of one level, 8 children); thread per parent cell.
+// One launch for the whole tree: a block starts at a brick whose children
+// have no children, restricts into it, and goes on to its parent if it is the
+// last of that brick's refined children to be done (a counter per brick, back
+// to zero for the next launch), so children come first as in the recursion
+// and no block waits.  A launch per level was 9 us of latency each.
+// grid = bricks whose children are all leaves; thread per parent cell.
 // ---------------------------------------------------------------------------
-__global__ void k_inject(Geom g, BrickTable bt, DevState st, const int* __restrict__ slots) {
-    const int p = slots[blockIdx.x];
-    const int c = blockIdx.y;
-    const int ch = bt.child[8 * p + c];
-    if (ch < 0) return;
-    const int nx = g.nx, gnx = g.gnx, bw = g.bw, half = nx / 2;
-    const int t = threadIdx.x;
-    if (t >= half * half * half) return;
-    const int a = t % half, bb = (t / half) % half, cc = t / (half * half);
-    const int i = bw + 2 * a, j = bw + 2 * bb, k = bw + 2 * cc;
-    const int i0 = bw + a + (c & 1) * half, j0 = bw + bb + ((c >> 1) & 1) * half, k0 = bw + cc + ((c >> 2) & 1) * half;
-    const double* C = st.U + (size_t)ch * g.ucount;
-    double* P = st.U + (size_t)p * g.ucount;
-    double u[NF_EULER];
+__global__ void __launch_bounds__(512) k_inject(Geom g, BrickTable bt, DevState st, const int* __restrict__ starts,
+                                                const int* __restrict__ refined, unsigned* done) {
+    __shared__ int s_next;
+    const int nx = g.nx, gnx = g.gnx, bw = g.bw, half = nx / 2, h3 = half * half * half;
+    int p = starts[blockIdx.x];
+    for (;;) {
+        double* P = st.U + (size_t)p * g.ucount;
+        for (int q = threadIdx.x; q < 8 * h3; q += blockDim.x) {
+            const int c = q / h3, t = q % h3;
+            const int ch = bt.child[8 * p + c];
+            if (ch < 0) continue;
+            const int a = t % half, bb = (t / half) % half, cc = t / (half * half);
+            const int i = bw + 2 * a, j = bw + 2 * bb, k = bw + 2 * cc;
+            const int i0 = bw + a + (c & 1) * half, j0 = bw + bb + ((c >> 1) & 1) * half,
+                      k0 = bw + cc + ((c >> 2) & 1) * half;
+            const double* C = st.U + (size_t)ch * g.ucount + cell_index(gnx, i, j, k);
+            double u[NF_EULER];
 #pragma unroll
-    for (int l = 0; l < NF_EULER; l++) {
-        const double* Cl = C + l * g.gnx3;
-        double s = 0.0;
-        s += Cl[cell_index(gnx, i + 0, j + 0, k + 0)];
-        s += Cl[cell_index(gnx, i + 1, j + 0, k + 0)];
-        s += Cl[cell_index(gnx, i + 0, j + 1, k + 0)];
-        s += Cl[cell_index(gnx, i + 1, j + 1, k + 0)];
-        s += Cl[cell_index(gnx, i + 0, j + 0, k + 1)];
-        s += Cl[cell_index(gnx, i + 1, j + 0, k + 1)];
-        s += Cl[cell_index(gnx, i + 0, j + 1, k + 1)];
-        s += Cl[cell_index(gnx, i + 1, j + 1, k + 1)];
-        u[l] = s * 0.125;
+            for (int l = 0; l < NF_EULER; l++) {
+                const double* Cl = C + l * g.gnx3;
+                // plain loads, although another block of this launch may have
+                // written the child: nothing reads these cells before this
+                // block does, so no line of them is in its SM's first cache
+                double s = 0.0;
+                s += Cl[0];
+                s += Cl[1];
+                s += Cl[gnx];
+                s += Cl[gnx + 1];
+                s += Cl[gnx * gnx];
+                s += Cl[gnx * gnx + 1];
+                s += Cl[gnx * gnx + gnx];
+                s += Cl[gnx * gnx + gnx + 1];
+                u[l] = s * 0.125;
+            }
+            st_floor(u, g.gamma, g.rho_floor, g.ei_floor);
+            const int dst = cell_index(gnx, i0, j0, k0);
+#pragma unroll
+            for (int l = 0; l < NF_EULER; l++) P[l * g.gnx3 + dst] = u[l];
+        }
+        const int up = bt.parent[p];
+        if (up < 0) return;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const bool last = atomicAdd(done + up, 1u) == (unsigned)refined[up] - 1u;
+            if (last) done[up] = 0u;
+            s_next = last ? up : -1;
+        }
+        __syncthreads();
+        p = s_next;
+        if (p < 0) return;
+        __threadfence();
     }
-    st_floor(u, g.gamma, g.rho_floor, g.ei_floor);
-    const int dst = cell_index(gnx, i0, j0, k0);
-#pragma unroll
-    for (int l = 0; l < NF_EULER; l++) P[l * g.gnx3 + dst] = u[l];
 }
 
 // ---------------------------------------------------------------------------
@@ -322,24 +407,11 @@ __global__ void k_prolong(Geom g, BrickTable bt, DevState st, const int* __restr
 
 // ---------------------------------------------------------------------------
 // CFL time step, Grid::max_dt (grid.cpp:422-483): largest face eigenvalue of
-// the reconstructed states over all three directions; per-brick dt out.
+// the reconstructed states of each direction, lam[3 b + d].  (The brick's
+// step, cfl / (max lam / h), is formed where the tree's is: cfl_step.)
 // ---------------------------------------------------------------------------
-template <int R>
-__global__ void k_max_dt(Geom g, DevState st, const int* __restrict__ slots, const double* __restrict__ hs,
-                         double* __restrict__ dt_out) {
-    const int b = slots[blockIdx.x];
-    const int npen = g.nx * g.nx;
+__device__ __forceinline__ void store_block_max(double lam, double* out) {
     __shared__ double red[32];
-    double lam = 0.0;
-    for (int t = threadIdx.x; t < 3 * npen; t += blockDim.x) {
-        const int d = t / npen, p = t % npen;
-        if (d == 0)
-            lam = max_eigen_pencil<0, R>(g, st, b, p, lam);
-        else if (d == 1)
-            lam = max_eigen_pencil<1, R>(g, st, b, p, lam);
-        else
-            lam = max_eigen_pencil<2, R>(g, st, b, p, lam);
-    }
     // block max (max is exact, order-free)
     for (int o = 16; o > 0; o >>= 1) lam = r_max(lam, __shfl_xor_sync(0xffffffffu, lam, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lam;
@@ -347,12 +419,24 @@ __global__ void k_max_dt(Geom g, DevState st, const int* __restrict__ slots, con
     if (threadIdx.x == 0) {
         double m = 0.0;
         for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) m = r_max(m, red[w]);
-        double dtinv = m / hs[b];
-        if (dtinv == 0.0) dtinv = 1.0E-10;
-        double dt = 1.0 / dtinv;
-        dt *= g.cfl;
-        dt_out[b] = dt;
+        *out = m;
     }
+}
+// grid = (bricks, 3 directions): staged pencils (flux_kernel.cuh), threads
+// rounded up to whole warps
+template <int R, bool LARGE>
+__global__ void __launch_bounds__(FluxBlock<LARGE>::THREADS, FluxBlock<LARGE>::PER_SM)
+    k_max_dt(Geom g, DevState st, const int* __restrict__ slots, double* __restrict__ lam_out) {
+    extern __shared__ double flux_smem[];
+    const int b = slots[blockIdx.x], d = blockIdx.y;
+    double lam;
+    if (d == 0)
+        lam = max_eigen_staged<0, R>(g, st, b, flux_smem);
+    else if (d == 1)
+        lam = max_eigen_staged<1, R>(g, st, b, flux_smem);
+    else
+        lam = max_eigen_staged<2, R>(g, st, b, flux_smem);
+    store_block_max(lam, lam_out + 3 * b + d);
 }
 
 // ---------------------------------------------------------------------------
@@ -410,36 +494,59 @@ void launch_ghost_fill(const Geom& g, const BrickTable& bt, const DevState& st, 
     if (n <= 0) return;
     launch_k(k_ghost_fill, dim3(n, 6), 128, 0, s, g, bt, st, slots);
 }
+void launch_ghost_fill_all(const Geom& g, const BrickTable& bt, const DevState& st, const int* slots, int n,
+                           cudaStream_t s) {
+    if (n <= 0) return;
+    const auto k = g.nx == 8 && g.bw == 2 ? k_ghost_fill_all<2, 8>
+                                          : (g.nx == 8 && g.bw == 3 ? k_ghost_fill_all<3, 8> : k_ghost_fill_all<0, 0>);
+    launch_k(k, dim3(n, 6), 128, 0, s, g, bt, st, slots);
+}
+namespace {
+template <int R, bool LARGE>
+void flux_fp64(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
+    const size_t smem = staged_smem<double, R>(g);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute((const void*)k_flux<R, LARGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_k(k_flux<R, LARGE>, dim3(n, 3), PENCIL_PARTS * g.nx * g.nx, smem, s, g, st, slots);
+}
+template <int R, bool LARGE>
+void max_dt_fp64(const Geom& g, const DevState& st, const int* slots, int n, double* lam, cudaStream_t s) {
+    const size_t smem = staged_smem<double, R>(g);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute((const void*)k_max_dt<R, LARGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int threads = (PENCIL_PARTS * g.nx * g.nx + 31) / 32 * 32;
+    launch_k(k_max_dt<R, LARGE>, dim3(n, 3), threads, smem, s, g, st, slots, lam);
+}
+}  // namespace
 void launch_flux(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
     if (n <= 0) return;
-    if (g.flux32) {
+    if (g.flux32)
         launch_flux_f32(g, st, slots, n, s);
-        return;
-    }
-    if (g.recon == RECON_PPM)
-        launch_k(k_flux<RECON_PPM>, n, 3 * g.nx * g.nx, 0, s, g, st, slots);
+    else if (g.recon == RECON_PPM)
+        (g.nx > 8 ? flux_fp64<RECON_PPM, true> : flux_fp64<RECON_PPM, false>)(g, st, slots, n, s);
     else
-        launch_k(k_flux<RECON_MINMOD>, n, 3 * g.nx * g.nx, 0, s, g, st, slots);
+        (g.nx > 8 ? flux_fp64<RECON_MINMOD, true> : flux_fp64<RECON_MINMOD, false>)(g, st, slots, n, s);
 }
-void launch_reflux(const Geom& g, const DevState& st, const RefluxItem* items, int n, cudaStream_t s) {
+void launch_reflux(const Geom& g, const BrickTable& bt, const DevState& st, const RefluxItem* items, int n,
+                   const unsigned char* fixes, unsigned* done, cudaStream_t s) {
     if (n <= 0) return;
     const int half = g.nx / 2;
-    launch_k(k_reflux, n, ((g.nf * half * half + 31) / 32) * 32, 0, s, g, st, items);
+    launch_k(k_reflux, n, ((g.nf * half * half + 31) / 32) * 32, 0, s, g, bt, st, items, fixes, done);
 }
 void launch_add_difs(const Geom& g, const DevState& st, const int* slots, int n, const double* hs, double dt,
-                     double beta, int gravity, cudaStream_t s, const double* dtp) {
+                     double beta, int gravity, int root, double* fo, cudaStream_t s, const double* dtp) {
     if (n <= 0) return;
-    launch_k(k_add_difs, n, 256, 0, s, g, st, slots, hs, dt, dtp, beta, gravity);
+    launch_k(k_add_difs, dim3(n + 1, (g.nx * g.nx * g.nx + 255) / 256), 256, 0, s, g, st, slots, hs, dt, dtp, beta,
+             gravity, root, fo);
 }
 void launch_flow_off(const Geom& g, const DevState& st, int root, double h, double dt, double beta, double* fo,
-                     cudaStream_t s, const double* dtp) {
-    launch_k(k_flow_off, 1, 32, 0, s, g, st, root, h, dt, dtp, beta, fo);
+                     cudaStream_t s) {
+    launch_k(k_flow_off, 1, 256, 0, s, g, st, root, h, dt, beta, fo);
 }
-void launch_inject(const Geom& g, const BrickTable& bt, const DevState& st, const int* slots, int n,
-                   cudaStream_t s) {
+void launch_inject(const Geom& g, const BrickTable& bt, const DevState& st, const int* starts, int n,
+                   const int* refined, unsigned* done, cudaStream_t s) {
     if (n <= 0) return;
-    const int half = g.nx / 2;
-    launch_k(k_inject, dim3(n, 8), ((half * half * half + 31) / 32) * 32, 0, s, g, bt, st, slots);
+    launch_k(k_inject, n, std::min(512, (g.nx * g.nx * g.nx + 31) / 32 * 32), 0, s, g, bt, st, starts, refined, done);
 }
 void launch_prolong(const Geom& g, const BrickTable& bt, const DevState& st, const int* slots, int n,
                     cudaStream_t s) {
@@ -447,13 +554,12 @@ void launch_prolong(const Geom& g, const BrickTable& bt, const DevState& st, con
     const int half = g.nx / 2;
     launch_k(k_prolong, n, ((half * half * half + 31) / 32) * 32, 0, s, g, bt, st, slots);
 }
-void launch_max_dt(const Geom& g, const DevState& st, const int* slots, int n, const double* hs, double* dt_out,
-                   cudaStream_t s) {
+void launch_max_dt(const Geom& g, const DevState& st, const int* slots, int n, double* lam, cudaStream_t s) {
     if (n <= 0) return;
     if (g.recon == RECON_PPM)
-        launch_k(k_max_dt<RECON_PPM>, n, 192, 0, s, g, st, slots, hs, dt_out);
+        (g.nx > 8 ? max_dt_fp64<RECON_PPM, true> : max_dt_fp64<RECON_PPM, false>)(g, st, slots, n, lam, s);
     else
-        launch_k(k_max_dt<RECON_MINMOD>, n, 192, 0, s, g, st, slots, hs, dt_out);
+        (g.nx > 8 ? max_dt_fp64<RECON_MINMOD, true> : max_dt_fp64<RECON_MINMOD, false>)(g, st, slots, n, lam, s);
 }
 void launch_refine_flags(const Geom& g, const DevState& st, const int* slots, int n, double thr,
                          unsigned char* flags, cudaStream_t s) {

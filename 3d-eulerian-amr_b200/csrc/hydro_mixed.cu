@@ -8,16 +8,27 @@
 namespace amr {
 
 template <int R>
-__global__ void k_flux_f32(Geom g, DevState st, const int* __restrict__ slots) {
-    flux_pencils<float, R>(g, st, slots[blockIdx.x]);
+__global__ void __launch_bounds__(FluxBlock<true>::THREADS, 2) k_flux_f32(Geom g, DevState st, const int* __restrict__ slots) {
+    extern __shared__ float flux_smem_f32[];
+    flux_staged<float, R>(g, st, slots[blockIdx.x], flux_smem_f32);
 }
+
+namespace {
+template <int R>
+void flux_fp32(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
+    const size_t smem = staged_smem<float, R>(g);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute((const void*)k_flux_f32<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_k(k_flux_f32<R>, dim3(n, 3), PENCIL_PARTS * g.nx * g.nx, smem, s, g, st, slots);
+}
+}  // namespace
 
 void launch_flux_f32(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
     if (n <= 0) return;
     if (g.recon == RECON_PPM)
-        launch_k(k_flux_f32<RECON_PPM>, n, 3 * g.nx * g.nx, 0, s, g, st, slots);
+        flux_fp32<RECON_PPM>(g, st, slots, n, s);
     else
-        launch_k(k_flux_f32<RECON_MINMOD>, n, 3 * g.nx * g.nx, 0, s, g, st, slots);
+        flux_fp32<RECON_MINMOD>(g, st, slots, n, s);
 }
 
 }  // namespace amr

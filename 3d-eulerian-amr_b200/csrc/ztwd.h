@@ -26,10 +26,13 @@ void launch_zt_ghost_fill(const Geom& g, const BrickTable& bt, const DevState& s
 // primitives + fluxes (+ face-averaged normal velocities)
 void launch_zt_flux(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P, const int* slots,
                     int n, int* err, cudaStream_t s);
+// largest eigenvalue of each direction, lam[3 slot + d]; nslots: slots in use
 void launch_zt_max_dt(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P, const int* slots,
-                      int n, double* dt_out, int* err, cudaStream_t s);
+                      int n, double* lam, int nslots, int* err, cudaStream_t s);
+// with the root's flow-off
 void launch_zt_add_difs(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P,
-                        const int* slots, int n, double dt, double beta, int* err, cudaStream_t s);
+                        const int* slots, int n, double dt, double beta, int* err, int root, double* fo,
+                        cudaStream_t s);
 void launch_zt_inject(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P,
                       const int* slots, int n, int* err, cudaStream_t s);
 void launch_zt_prolong(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P,

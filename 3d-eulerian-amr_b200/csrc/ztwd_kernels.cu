@@ -12,6 +12,7 @@
 // first such status is kept in an error word and the host returns
 // AMR_ERR_RANGE.
 #include "euler_state.cuh"
+#include "flow_off.cuh"
 #include "flux_kernel.cuh"
 #include "launch.cuh"
 #include "poisson_ops.cuh"
@@ -133,7 +134,7 @@ __global__ void k_zt_prim(Geom g, BrickTable bt, DevState st, ZtwdPar P, const i
     const int gnx = g.gnx, bw = g.bw;
     const double* U = st.U + (size_t)b * g.ucount;
     double* W = st.W + (size_t)b * g.ucount;
-    for (int t = threadIdx.x; t < g.gnx3; t += blockDim.x) {
+    for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < g.gnx3; t += gridDim.y * blockDim.x) {
         const int i = t % gnx, j = (t / gnx) % gnx, k = t / (gnx * gnx);
         const int out = (i < bw || i >= gnx - bw) + (j < bw || j >= gnx - bw) + (k < bw || k >= gnx - bw);
         if (out > 1) continue;  // edge and corner ghosts: never read
@@ -245,7 +246,9 @@ __device__ __forceinline__ void face_X(const Geom& g, const BrickTable& bt, int 
 // with PPM, the face states to_con'd at the face centre, p and cs from one
 // EOS call per face state, and the face-averaged normal velocity.
 // Binary::compute_*_flux's adjust_rho_fluxes (binary.cpp:1171-1235) has an
-// empty body (state_ztwd.cpp:445-480).  Block = one brick, thread per face.
+// empty body (state_ztwd.cpp:445-480).  grid = (bricks, faces / 128), one face
+// a thread: a block per brick left 33 bricks on 33 of 148 SMs (655 us) and 309
+// bricks in two waves.
 // T = double: the plain form.  T = float: the mixed form's reconstruction,
 // to_con and KT combination in FP32 from the FP64 primitives, the EOS in
 // FP64 (zt_eos_of), the fluxes and face velocities stored in FP64 for the
@@ -258,7 +261,8 @@ __global__ void __launch_bounds__(128) k_zt_flux(Geom g, BrickTable bt, DevState
     const int nx = g.nx, bw = g.bw;
     const int fstride = nx * nx * (nx + 1);
     const double* W = st.W + (size_t)b * g.ucount;
-    for (int q = threadIdx.x; q < 3 * fstride; q += blockDim.x) {
+    const int q = blockIdx.y * blockDim.x + threadIdx.x;
+    if (q < 3 * fstride) {
         const int d = q / fstride, r = q % fstride;
         int fi, t1, t2, base, stride;
         face_decode(d, nx, r, fi, t1, t2);
@@ -295,18 +299,20 @@ __global__ void __launch_bounds__(128) k_zt_flux(Geom g, BrickTable bt, DevState
     }
 }
 
-// Grid::max_dt (grid.cpp:422-483) with the ZTWD eigenvalues |v| + cs
+// Grid::max_dt (grid.cpp:422-483) with the ZTWD eigenvalues |v| + cs: the
+// largest of each direction, lam_out[3 b + d] (zero before the launch; the
+// values are not negative, so their bits order as integers).  grid =
+// (bricks, faces of a direction / 128, 3 directions).
 __global__ void __launch_bounds__(128) k_zt_max_dt(Geom g, BrickTable bt, DevState st, ZtwdPar P,
-                                                   const int* __restrict__ slots, double* __restrict__ dt_out,
+                                                   const int* __restrict__ slots, double* __restrict__ lam_out,
                                                    int* err) {
     const int b = slots[blockIdx.x];
     const int nx = g.nx, bw = g.bw;
     const int fstride = nx * nx * (nx + 1);
     const double* W = st.W + (size_t)b * g.ucount;
-    __shared__ double red[32];
     double lam = 0.0;
-    for (int q = threadIdx.x; q < 3 * fstride; q += blockDim.x) {
-        const int d = q / fstride, r = q % fstride;
+    const int d = blockIdx.z, r = blockIdx.y * blockDim.x + threadIdx.x;
+    if (r < fstride) {
         int fi, t1, t2, base, stride;
         face_decode(d, nx, r, fi, t1, t2);
         pencil_of(g, d, t1, t2, base, stride);
@@ -324,17 +330,9 @@ __global__ void __launch_bounds__(128) k_zt_max_dt(Geom g, BrickTable bt, DevSta
         lam = zmax(lam, zmax(al, ar));
     }
     for (int o = 16; o > 0; o >>= 1) lam = zmax(lam, __shfl_xor_sync(0xffffffffu, lam, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lam;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) m = zmax(m, red[w]);
-        double dtinv = m / bt.h[b];
-        if (dtinv == 0.0) dtinv = 1.0E-10;
-        double dt = 1.0 / dtinv;
-        dt *= g.cfl;
-        dt_out[b] = dt;
-    }
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(lam_out + 3 * b + d),
+                  (unsigned long long)__double_as_longlong(lam));
 }
 
 // ---------------------------------------------------------------------------
@@ -342,11 +340,16 @@ __global__ void __launch_bounds__(128) k_zt_max_dt(Geom g, BrickTable bt, DevSta
 // of Binary::add_difs (binary.cpp:205-245: gravity source from the mean face
 // forces, -p div u from the face-averaged velocities, D[pot] = D[T] = 0),
 // then Grid::add_difs (grid.cpp:406-420: State::source, RK combine,
-// State::floor).  Block = one brick, thread per interior cell.
+// State::floor).  grid = (bricks, cells / 128) + the root's flow-off in the
+// last block of the first row; thread per interior cell.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_zt_add_difs(Geom g, BrickTable bt, DevState st, ZtwdPar P,
                                                      const int* __restrict__ slots, double dt, double beta,
-                                                     int* err) {
+                                                     int* err, int root, double* fo) {
+    if (blockIdx.x == gridDim.x - 1) {
+        if (blockIdx.y == 0) flow_off_block(g, st, root, bt.h[root], dt, beta, fo);
+        return;
+    }
     const int b = slots[blockIdx.x];
     const int nx = g.nx, gnx = g.gnx, bw = g.bw, pnx = g.pnx;
     const int npen = nx * nx, fstride = npen * (nx + 1);
@@ -361,7 +364,8 @@ __global__ void __launch_bounds__(128) k_zt_add_difs(Geom g, BrickTable bt, DevS
     double* U = st.U + (size_t)b * g.ucount;
     const double* U0 = st.U0 + (size_t)b * g.ucount;
     const size_t pb = (size_t)b * g.pnx3;
-    for (int t = threadIdx.x; t < nx * nx * nx; t += blockDim.x) {
+    const int t = blockIdx.y * blockDim.x + threadIdx.x;
+    if (t < nx * nx * nx) {
         const int i = t % nx, j = (t / nx) % nx, k = t / npen;
         double D[ZT_NF];
         const int a0 = flux_index(0, nx, i, j, k), a1 = flux_index(0, nx, i + 1, j, k);
@@ -550,25 +554,35 @@ void launch_zt_ghost_fill(const Geom& g, const BrickTable& bt, const DevState& s
     if (n <= 0) return;
     launch_k(k_zt_ghost_fill, dim3(n, 6), 128, 0, s, g, bt, st, P, slots);
 }
+namespace {
+void launch_zt_prim(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P, const int* slots,
+                    int n, cudaStream_t s) {
+    launch_k(k_zt_prim, dim3(n, (g.gnx3 + 255) / 256), 256, 0, s, g, bt, st, P, slots);
+}
+}  // namespace
 void launch_zt_flux(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P, const int* slots,
                     int n, int* err, cudaStream_t s) {
     if (n <= 0) return;
-    launch_k(k_zt_prim, n, 256, 0, s, g, bt, st, P, slots);
+    launch_zt_prim(g, bt, st, P, slots, n, s);
+    const dim3 grid(n, (3 * g.nx * g.nx * (g.nx + 1) + 127) / 128);
     if (g.flux32)
-        launch_k(k_zt_flux<float>, n, 128, 0, s, g, bt, st, P, slots, err);
+        launch_k(k_zt_flux<float>, grid, 128, 0, s, g, bt, st, P, slots, err);
     else
-        launch_k(k_zt_flux<double>, n, 128, 0, s, g, bt, st, P, slots, err);
+        launch_k(k_zt_flux<double>, grid, 128, 0, s, g, bt, st, P, slots, err);
 }
 void launch_zt_max_dt(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P, const int* slots,
-                      int n, double* dt_out, int* err, cudaStream_t s) {
+                      int n, double* lam, int nslots, int* err, cudaStream_t s) {
     if (n <= 0) return;
-    launch_k(k_zt_prim, n, 256, 0, s, g, bt, st, P, slots);
-    launch_k(k_zt_max_dt, n, 128, 0, s, g, bt, st, P, slots, dt_out, err);
+    launch_zt_prim(g, bt, st, P, slots, n, s);
+    cudaMemsetAsync(lam, 0, sizeof(double) * 3 * (size_t)nslots, s);
+    launch_k(k_zt_max_dt, dim3(n, (g.nx * g.nx * (g.nx + 1) + 127) / 128, 3), 128, 0, s, g, bt, st, P, slots, lam, err);
 }
 void launch_zt_add_difs(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P,
-                        const int* slots, int n, double dt, double beta, int* err, cudaStream_t s) {
+                        const int* slots, int n, double dt, double beta, int* err, int root, double* fo,
+                        cudaStream_t s) {
     if (n <= 0) return;
-    launch_k(k_zt_add_difs, n, 128, 0, s, g, bt, st, P, slots, dt, beta, err);
+    launch_k(k_zt_add_difs, dim3(n + 1, (g.nx * g.nx * g.nx + 127) / 128), 128, 0, s, g, bt, st, P, slots, dt, beta,
+             err, root, fo);
 }
 void launch_zt_inject(const Geom& g, const BrickTable& bt, const DevState& st, const ZtwdPar& P,
                       const int* slots, int n, int* err, cudaStream_t s) {
