@@ -81,13 +81,28 @@ __device__ constexpr int OT[9] = {0, 1, 2, 0, 0, 1, 1, 2, 2};
 
 }  // namespace
 
-// helmholtz_eos (helmeos.cpp:164-421) at one point in code units.
+// Four doubles of one 32-byte sector in one load (sm_100): a point's table
+// loads go to addresses of its own, so what they cost is the number of load
+// instructions, each one line a lane.
+struct Quad {
+    double a, b, c, d;
+};
+__device__ __forceinline__ Quad load_quad(const double* p) {
+    Quad q;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.a), "=d"(q.b), "=d"(q.c), "=d"(q.d) : "l"(p));
+    return q;
+}
+
+// helmholtz_eos (helmeos.cpp:164-421) at one point in code units.  S: with the
+// entropy and its derivative (else they are left as they are).
+template <bool S = true>
 __device__ __forceinline__ void helm_point(const HelmTable& H, double rho_code, double T_code, double abar, double zbar,
                            HelmPoint& o) {
     const double den = rho_code * H.u.f_rho;  // eos_from_code (helmeos.cpp:153-162)
     const double Tc = T_code * H.u.f_T;
-    o.rho = den / H.u.f_rho;  // eos_to_code applied to the inputs (helmeos.cpp:142-151)
-    o.T = Tc / H.u.f_T;
+    // eos_to_code applied to the inputs (helmeos.cpp:142-151)
+    o.rho = H.u.cgs ? den : den / H.u.f_rho;
+    o.T = H.u.cgs ? Tc : Tc / H.u.f_T;
     const double temp = hmax(Tc, HELM_TMIN);
     const double ytot1 = 1.0 / abar;
     const double ye = hmax(1.0 - 16, ytot1 * zbar);  // the reference writes 1.0d - 16
@@ -102,19 +117,23 @@ __device__ __forceinline__ void helm_point(const HelmTable& H, double rho_code, 
     const double eion = 1.5 * pion * deni;
     const double deiondt = 1.5 * dpiondt * deni;
     // Sackur-Tetrode ion entropy
-    double x = abar * abar * sqrt(abar) * deni / C_AVO;
-    const double s = ((2.0 * C_PI * C_AMU * C_KERG) / (C_H * C_H)) * temp;
-    const double z = x * s * sqrt(s);
-    const double y = log(z);
-    const double tempi = 1.0 / temp;
-    const double sion = (pion * deni + eion) * tempi + C_KERG * C_AVO * ytot1 * y;
-    const double dsiondt = (dpiondt * deni + deiondt) * tempi - (pion * deni + eion) * tempi * tempi +
-                           1.5 * C_KERG * C_AVO * tempi * ytot1;
+    double x, sion = 0.0, dsiondt = 0.0;
+    if constexpr (S) {
+        x = abar * abar * sqrt(abar) * deni / C_AVO;
+        const double s = ((2.0 * C_PI * C_AMU * C_KERG) / (C_H * C_H)) * temp;
+        const double z = x * s * sqrt(s);
+        const double y = log(z);
+        const double tempi = 1.0 / temp;
+        sion = (pion * deni + eion) * tempi + C_KERG * C_AVO * ytot1 * y;
+        dsiondt = (dpiondt * deni + deiondt) * tempi - (pion * deni + eion) * tempi * tempi +
+                  1.5 * C_KERG * C_AVO * tempi * ytot1;
+    }
     // electron-positron section: enter the table with ye*den
     const double din = ye * den;
     if ((temp > H.t_last) || (temp < H.t_first) || (din > H.d_last) || (din < H.d_first)) {
         o.status = 1;  // the reference aborts here
-        o.p = o.e = o.cs = o.cv = o.s = o.dsdt = __longlong_as_double(0x7ff8000000000000LL);
+        o.p = o.e = o.cs = o.cv = __longlong_as_double(0x7ff8000000000000LL);
+        if constexpr (S) o.s = o.dsdt = o.p;
         return;
     }
     int jat = int((log10(temp) - H.tlo) * H.tstpi) + 1;
@@ -123,29 +142,28 @@ __device__ __forceinline__ void helm_point(const HelmTable& H, double rho_code, 
     iat = (int)hmax(1, hmin(iat, HELM_IMAX - 1));
     --jat;
     --iat;
-    const double* tj = H.tj + 8 * jat;
-    const double* di = H.di + 8 * iat;
-    const double t_j = __ldg(tj + 0), dt = __ldg(tj + 1), dt2 = __ldg(tj + 2), dti = __ldg(tj + 3),
-                 dt2i = __ldg(tj + 4);
-    const double d_i = __ldg(di + 0), dd = __ldg(di + 1), dd2 = __ldg(di + 2), ddi = __ldg(di + 3),
-                 dd2i = __ldg(di + 4);
+    const Quad nt = load_quad(H.tj + 4 * jat), nd = load_quad(H.di + 4 * iat);
+    const double t_j = nt.a, dt = nt.b, dt2 = dt * dt, dti = nt.c, dt2i = nt.d;
+    const double d_i = nd.a, dd = nd.b, dd2 = dd * dd, ddi = nd.c, dd2i = nd.d;
     const double xt = hmax((temp - t_j) * dti, 0.0);
     const double xd = hmax((din - d_i) * ddi, 0.0);
     AxisWeights wt, wd;
     axis_weights(xt, dt, dt2, dti, dt2i, wt);
     axis_weights(xd, dd, dd2, ddi, dd2i, wd);
-    // node values of the four corners: rows j and j+1, each a 20-double run
-    // (two nodes of 10) starting at node (iat, row)
-    const double2* r0 = reinterpret_cast<const double2*>(H.node + ((size_t)jat * HELM_IMAX + iat) * HELM_NODE);
-    const double2* r1 = reinterpret_cast<const double2*>(H.node + ((size_t)(jat + 1) * HELM_IMAX + iat) * HELM_NODE);
+    // node values of the four corners: rows j and j+1, two nodes each
+    const double* r0 = H.node + ((size_t)jat * HELM_IMAX + iat) * HELM_NODE;
+    const double* r1 = r0 + (size_t)HELM_IMAX * HELM_NODE;
     double v0[2 * HELM_NODE], v1[2 * HELM_NODE];
 #pragma unroll
-    for (int q = 0; q < HELM_NODE; q++) {
-        const double2 a = __ldg(r0 + q), b = __ldg(r1 + q);
-        v0[2 * q] = a.x;
-        v0[2 * q + 1] = a.y;
-        v1[2 * q] = b.x;
-        v1[2 * q + 1] = b.y;
+    for (int q = 0; q < 2 * HELM_NODE; q += HELM_NODE) {
+#pragma unroll
+        for (int u = 0; u < 8; u += 4) {
+            const Quad a = load_quad(r0 + q + u), b = load_quad(r1 + q + u);
+            v0[q + u] = a.a, v0[q + u + 1] = a.b, v0[q + u + 2] = a.c, v0[q + u + 3] = a.d;
+            v1[q + u] = b.a, v1[q + u + 1] = b.b, v1[q + u + 2] = b.c, v1[q + u + 3] = b.d;
+        }
+        v0[q + 8] = __ldg(r0 + q + 8);
+        v1[q + 8] = __ldg(r1 + q + 8);
     }
     // the six biquintic sums (helmeos.cpp:327-354), term by term in order
     double free = 0.0, df_d = 0.0, df_t = 0.0, df_dd = 0.0, df_tt = 0.0, df_dt = 0.0;
@@ -196,12 +214,25 @@ __device__ __forceinline__ void helm_point(const HelmTable& H, double rho_code, 
     } else {
         cs = sqrt(x);
     }
-    o.p = p / H.u.f_p;
-    o.e = e / H.u.f_e;
-    o.cs = cs / H.u.f_cs;
-    o.cv = cv / H.u.f_cv;
-    o.s = sv / H.u.f_s;
-    o.dsdt = dsdt / H.u.f_dsdt;
+    if (H.u.cgs) {
+        o.p = p;
+        o.e = e;
+        o.cs = cs;
+        o.cv = cv;
+        if constexpr (S) {
+            o.s = sv;
+            o.dsdt = dsdt;
+        }
+    } else {
+        o.p = p / H.u.f_p;
+        o.e = e / H.u.f_e;
+        o.cs = cs / H.u.f_cs;
+        o.cv = cv / H.u.f_cv;
+        if constexpr (S) {
+            o.s = sv / H.u.f_s;
+            o.dsdt = dsdt / H.u.f_dsdt;
+        }
+    }
 }
 
 // helmholtz_compute_T (helmeos.cpp:436-486) at one point: Newton on e(T) (or

@@ -49,6 +49,8 @@ HelmUnits make_units(double cm, double g, double s, double K) {
     u.f_rho = g / std::pow(cm, 3);
     u.f_s = erg / K / g;
     u.f_dsdt = erg / K / K / g;
+    u.cgs = u.f_p == 1.0 && u.f_e == 1.0 && u.f_T == 1.0 && u.f_cs == 1.0 && u.f_cv == 1.0 && u.f_rho == 1.0 &&
+            u.f_s == 1.0 && u.f_dsdt == 1.0;
     return u;
 }
 
@@ -125,29 +127,27 @@ int helm_create(const char* path, helm_ctx** out) {
     const double tlo = 3.0, thi = 13.0, dlo = -12.0, dhi = 15.0;
     const double tstp = (thi - tlo) / double(HELM_JMAX - 1);
     const double dstp = (dhi - dlo) / double(HELM_IMAX - 1);
-    std::vector<double> t(HELM_JMAX), d(HELM_IMAX), tj((size_t)HELM_JMAX * 8, 0.0), di((size_t)HELM_IMAX * 8, 0.0);
+    std::vector<double> t(HELM_JMAX), d(HELM_IMAX), tj((size_t)HELM_JMAX * 4, 0.0), di((size_t)HELM_IMAX * 4, 0.0);
     for (int j = 0; j < HELM_JMAX; j++) t[j] = std::pow(10.0, tlo + j * tstp);
     for (int i = 0; i < HELM_IMAX; i++) d[i] = std::pow(10.0, dlo + i * dstp);
     for (int j = 0; j < HELM_JMAX; j++) {
-        tj[8 * j] = t[j];
+        tj[4 * j] = t[j];
         if (j < HELM_JMAX - 1) {
             const double dth = t[j + 1] - t[j];
             const double dt2 = dth * dth;
-            tj[8 * j + 1] = dth;
-            tj[8 * j + 2] = dt2;
-            tj[8 * j + 3] = 1.0 / dth;
-            tj[8 * j + 4] = 1.0 / dt2;
+            tj[4 * j + 1] = dth;
+            tj[4 * j + 2] = 1.0 / dth;
+            tj[4 * j + 3] = 1.0 / dt2;
         }
     }
     for (int i = 0; i < HELM_IMAX; i++) {
-        di[8 * i] = d[i];
+        di[4 * i] = d[i];
         if (i < HELM_IMAX - 1) {
             const double dd = d[i + 1] - d[i];
             const double dd2 = dd * dd;
-            di[8 * i + 1] = dd;
-            di[8 * i + 2] = dd2;
-            di[8 * i + 3] = 1.0 / dd;
-            di[8 * i + 4] = 1.0 / dd2;
+            di[4 * i + 1] = dd;
+            di[4 * i + 2] = 1.0 / dd;
+            di[4 * i + 3] = 1.0 / dd2;
         }
     }
     auto fail = [&](cudaError_t e, const char* what) {

@@ -7,18 +7,19 @@
 
 namespace amr {
 
-constexpr int HELM_NODE = 10;  // doubles per table node (9 values + pad)
+constexpr int HELM_NODE = 12;  // doubles per table node (9 values, padded so that every node starts a 32-byte sector)
 
 // code <- cgs factors of helmholtz_set_cgs_units / eos_from_code
 // (helmeos.cpp:132-162): x_code = x_cgs / f_x
 struct HelmUnits {
     double f_p, f_e, f_T, f_cs, f_cv, f_rho, f_s, f_dsdt;
+    int cgs;  // every factor is 1: nothing to divide by
 };
 
 struct HelmTable {
     const double* node;  // [JMAX][IMAX][HELM_NODE]
-    const double* tj;    // [JMAX][8]: t, dt, dt^2, 1/dt, 1/dt^2
-    const double* di;    // [IMAX][8]: d, dd, dd^2, 1/dd, 1/dd^2
+    const double* tj;    // [JMAX][4]: t, dt, 1/dt, 1/dt^2
+    const double* di;    // [IMAX][4]: d, dd, 1/dd, 1/dd^2
     double tlo, tstpi, dlo, dstpi;
     double t_first, t_last, d_first, d_last;
     HelmUnits u;
