@@ -1037,8 +1037,7 @@ int fused_setup(amr_ctx* c) {
 
 }  // namespace
 
-// amr_sub_step of the Euler driver as one persistent launch (plus the root's
-// flow-off): ghost zones, fluxes, coarse-fine corrections and the RK
+// amr_sub_step of the Euler driver as one persistent launch: ghost zones, fluxes, coarse-fine corrections and the RK
 // combination per brick, the result written to the second state array which
 // then becomes the state.  Interiors are bitwise those of amr_sub_step (FP64
 // form); the ghost zones of the new state are not filled.
@@ -1075,6 +1074,7 @@ int amr_fused_sub_step(amr_ctx* c, double dt, double beta, int blocks_per_sm) {
     a.Fx = c->st.Fx;
     a.Fy = c->st.Fy;
     a.Fz = c->st.Fz;
+    a.fo = c->d_fo;
     a.err = reinterpret_cast<int*>(c->d_fctl + 1);
     a.wait_limit = (unsigned long long)c->fused_wait_limit;
     cudaError_t e;
@@ -1086,10 +1086,6 @@ int amr_fused_sub_step(amr_ctx* c, double dt, double beta, int blocks_per_sm) {
     if (e != cudaSuccess) {
         c->err = std::string("fused substep launch: ") + cudaGetErrorString(e);
         return AMR_ERR_CUDA;
-    }
-    {
-        ProfScope ps_(c->prof, KC_ADD_DIFS, c->stream);
-        launch_flow_off(c->geom, c->st, c->tree.root()->slot, c->tree.root()->h, dt, beta, c->d_fo, c->stream);
     }
     std::swap(c->st.U, c->d_U1);
     for (Node* n : c->order) n->age++;  // GridNode::add_difs, grid_node.cpp:338

@@ -21,6 +21,7 @@
 // so with FT = double the result is bitwise that of amr_sub_step.
 #pragma once
 
+#include "flow_off.cuh"
 #include "flux_kernel.cuh"
 #include "hydro_cell.cuh"
 #include "hydro_fused.h"
@@ -40,11 +41,14 @@ __device__ __forceinline__ void fused_wait(const FusedArgs& A, int child) {
     __threadfence();
 }
 
-// Block layout: 512 threads; per brick the "cross" -- the 8^3 interior and
-// the six 2-deep ghost slabs the dimension-split stencil reads -- is held in
-// shared memory as primitives (FT), and one direction's 9 x 64 face fluxes
-// (FP64) at a time.
-constexpr int FUSED_BLOCK = 256;  // two cells per thread in the per-cell phases
+// Block layout: per brick the "cross" -- the 8^3 interior and the six 2-deep
+// ghost slabs the dimension-split stencil reads -- is held in shared memory as
+// primitives (FT), and one direction's 576 face fluxes (FP64) at a time.  288
+// threads take the faces in two full rounds; 256 left a third round with a
+// quarter of them.  Faces are numbered so that neighbouring threads read and
+// write neighbouring words in every direction (with the pencil fastest in x,
+// two thirds of the shared-memory wavefronts were bank conflicts).
+constexpr int FUSED_BLOCK = 288;
 constexpr int CROSS = 512 + 6 * 2 * 64;  // interior + ghost slabs
 constexpr int FACES = 9 * 64;            // faces of one direction
 
@@ -57,6 +61,21 @@ __device__ __forceinline__ int cross_index(int d, int n, int t1, int t2) {
     const int x = d == 0 ? i : t1, y = d == 1 ? i : (d == 0 ? t1 : t2), z = d == 2 ? i : t2;
     return (z * 8 + y) * 8 + x;
 }
+// face number q of direction d <-> its position fi along d and its pencil
+__device__ __forceinline__ void face_of(int d, int q, int& fi, int& t1, int& t2) {
+    if (d == 0) {
+        fi = q % 9, t1 = (q / 9) % 8, t2 = q / 72;
+    } else if (d == 1) {
+        t1 = q % 8, fi = (q / 8) % 9, t2 = q / 72;
+    } else {
+        t1 = q % 8, t2 = (q / 8) % 8, fi = q / 64;
+    }
+}
+// the lower face of cell (x, y, z) along d, and the step to its upper face
+__device__ __forceinline__ int cell_face(int d, int x, int y, int z) {
+    return d == 0 ? (z * 8 + y) * 9 + x : (d == 1 ? z * 72 + y * 8 + x : (z * 8 + y) * 8 + x);
+}
+__device__ __forceinline__ int face_step(int d) { return d == 0 ? 1 : (d == 1 ? 8 : 64); }
 
 template <typename FT>
 __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, FT* P, double* Fs) {
@@ -64,22 +83,21 @@ __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, F
     const int nx = 8, gnx = 12, bw = 2, npen = 64, half = 4;
     const int tid = threadIdx.x;
     // (a) the cross as primitives: interior cells, then ghost cells resolved
-    //     as the level-ordered ghost fill would have set them
+    //     as the level-ordered ghost fill would have set them (one call: its
+    //     code is long, and the block runs through all of this kernel's)
+#pragma unroll 1
     for (int q = tid; q < CROSS; q += FUSED_BLOCK) {
-        Cell6 u;
-        if (q < 512) {
-            cell_load(A.Uin, A.g.ucount, gnx, A.g.gnx3, b, q % 8 + bw, (q / 8) % 8 + bw, q / 64 + bw, u);
-        } else {
-            const int r = q - 512, t1 = r % 8 + bw, t2 = (r / 8) % 8 + bw, depth = (r / 64) % 2, face = r / 128;
+        int x = q % 8 + bw, y = (q / 8) % 8 + bw, z = q / 64 + bw;
+        if (q >= 512) {
+            const int r = q - 512, t1 = x, t2 = (r / 8) % 8 + bw, depth = (r / 64) % 2, face = r / 128;
             const int ax = face >> 1;
             const int n = (face & 1) ? gnx - bw + depth : depth;
-            if (ax == 0)
-                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, n, t1, t2, u, A.err);
-            else if (ax == 1)
-                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, t1, n, t2, u, A.err);
-            else
-                ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, t1, t2, n, u, A.err);
+            x = ax == 0 ? n : t1;
+            y = ax == 1 ? n : (ax == 0 ? t1 : t2);
+            z = ax == 2 ? n : t2;
         }
+        Cell6 u;
+        ghost_cell<1, 2, 12>(A.g, A.bt, A.Uin, b, x, y, z, u, A.err);
         FT w[NF_EULER];
 #pragma unroll
         for (int l = 0; l < NF_EULER; l++) w[l] = (FT)u.v[l];
@@ -93,20 +111,23 @@ __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, F
     const unsigned char pm = A.pubmask[b];
     double* pubb = A.pub + (size_t)b * 6 * NF_EULER * npen;
     const int* rg = vr >= 0 ? A.vranges + 4 * vr : nullptr;
-    double D[2][NF_EULER];  // this thread's cells tid, tid + 256: flux differences, x then y then z
+    double D[2][NF_EULER];  // this thread's cells tid, tid + 288: flux differences, x then y then z
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
         for (int l = 0; l < NF_EULER; l++) D[h][l] = 0.0;
     // unrolled: the direction is a compile-time constant in each copy, so the
     // state arrays indexed by it (normal velocity, normal momentum flux) stay
-    // in registers
+    // in registers (one copy with the direction chosen by selects is smaller
+    // but spills: 449 against 424 us for 2505 bricks)
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         // (b) face fluxes of direction d, one thread per face
+#pragma unroll 1
         for (int q = tid; q < FACES; q += FUSED_BLOCK) {
-            const int p = q % npen, fi = q / npen;
-            const int t1 = p % nx, t2 = p / nx;
+            int fi, t1, t2;
+            face_of(d, q, fi, t1, t2);
+            const int p = t2 * nx + t1;
             FT w[4][NF_EULER];  // cells f-2 .. f+1 (f = fi + bw)
 #pragma unroll
             for (int m = 0; m < 4; m++) {
@@ -172,12 +193,10 @@ __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, F
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int cc = tid + h * FUSED_BLOCK;
-                const int x = cc % 8, y = (cc / 8) % 8, z = cc / 64;
-                const int i = d == 0 ? x : (d == 1 ? y : z);
-                const int p = d == 0 ? z * 8 + y : (d == 1 ? z * 8 + x : y * 8 + x);
+                if (cc >= 512) break;
+                const int lo = cell_face(d, cc % 8, (cc / 8) % 8, cc / 64), up = lo + face_step(d);
 #pragma unroll
-                for (int l = 0; l < NF_EULER; l++)
-                    D[h][l] -= (Fs[l * FACES + (i + 1) * npen + p] - Fs[l * FACES + i * npen + p]) * hinv;
+                for (int l = 0; l < NF_EULER; l++) D[h][l] -= (Fs[l * FACES + up] - Fs[l * FACES + lo]) * hinv;
             }
         }
         __syncthreads();
@@ -190,6 +209,7 @@ __device__ __forceinline__ void fused_brick(const FusedArgs& A, int b, int vr, F
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int cc = tid + h * FUSED_BLOCK;
+        if (cc >= 512) break;
         const int x = cc % 8, y = (cc / 8) % 8, z = cc / 64;
         const int ci = cell_index(gnx, x + bw, y + bw, z + bw);
         const double* U = A.Uin + (size_t)b * g.ucount;
@@ -218,8 +238,11 @@ __global__ void __launch_bounds__(FUSED_BLOCK, 2) k_substep_fused(FusedArgs A) {
         __syncthreads();
         const int w = s_item;
         if (w >= A.nwork) break;
-        fused_brick<FT>(A, A.work[w].x, A.work[w].y, P, Fs);
+        const int b = A.work[w].x;
+        fused_brick<FT>(A, b, A.work[w].y, P, Fs);
         __syncthreads();
+        // the root's fluxes are this block's own: their flow-off with them
+        if (b == A.root) flow_off_block(A.g, DevState{.Fx = A.Fx, .Fy = A.Fy, .Fz = A.Fz}, b, A.bt.h[b], A.dt, A.beta, A.fo);
     }
 }
 

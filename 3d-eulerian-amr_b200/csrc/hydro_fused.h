@@ -27,6 +27,7 @@ struct FusedArgs {
     double* Fx;  // the root's face fluxes (for the domain flow-off)
     double* Fy;
     double* Fz;
+    double* fo;  // FO, FO0 of the root
     int* err;  // bit 0: a wait for a child ran out; bit 1: ghost chain too deep
     unsigned long long wait_limit;  // polls of one wait for a child's faces before bit 0 is set
 };

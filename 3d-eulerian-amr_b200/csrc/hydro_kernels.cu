@@ -291,12 +291,6 @@ __global__ void __launch_bounds__(256) k_add_difs(Geom g, DevState st, const int
     }
 }
 
-// The root's flow-off by itself (the fused substep).
-__global__ void __launch_bounds__(256) k_flow_off(Geom g, DevState st, int root, double h, double dt, double beta,
-                                                  double* fo) {
-    flow_off_block(g, st, root, h, dt, beta, fo);
-}
-
 // ---------------------------------------------------------------------------
 // Restriction, GridNode::inject_from_children (grid_node.cpp:1035-1074):
 // covered parent cell := mean of its 8 child cells, then floor.
@@ -538,10 +532,6 @@ void launch_add_difs(const Geom& g, const DevState& st, const int* slots, int n,
     if (n <= 0) return;
     launch_k(k_add_difs, dim3(n + 1, (g.nx * g.nx * g.nx + 255) / 256), 256, 0, s, g, st, slots, hs, dt, dtp, beta,
              gravity, root, fo);
-}
-void launch_flow_off(const Geom& g, const DevState& st, int root, double h, double dt, double beta, double* fo,
-                     cudaStream_t s) {
-    launch_k(k_flow_off, 1, 256, 0, s, g, st, root, h, dt, beta, fo);
 }
 void launch_inject(const Geom& g, const BrickTable& bt, const DevState& st, const int* starts, int n,
                    const int* refined, unsigned* done, cudaStream_t s) {

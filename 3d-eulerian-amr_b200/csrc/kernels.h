@@ -25,8 +25,6 @@ void launch_reflux(const Geom& g, const BrickTable& bt, const DevState& st, cons
 // memory (captured graphs)
 void launch_add_difs(const Geom& g, const DevState& st, const int* slots, int n, const double* hs, double dt,
                      double beta, int gravity, int root, double* fo, cudaStream_t s, const double* dtp = nullptr);
-void launch_flow_off(const Geom& g, const DevState& st, int root, double h, double dt, double beta, double* fo,
-                     cudaStream_t s);
 // whole tree: starts = bricks whose children are all leaves, refined[slot] =
 // children of a brick that have children, done[slot] zero between launches
 void launch_inject(const Geom& g, const BrickTable& bt, const DevState& st, const int* starts, int n,
