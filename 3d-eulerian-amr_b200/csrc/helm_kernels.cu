@@ -22,7 +22,7 @@ namespace {
 // bounds it: FP64 issue (about 900 operations a point, 0.8 ms for 2^24 points
 // at 64 a clock and SM, 67% busy), and before the 32-byte table loads the
 // first cache's gathers (30 load instructions a point, one line a lane each;
-// 14 now).  2^24 points to p, e, cs in cgs: 1.62 -> 1.11 ms.  Four blocks an
+// 14 now).  2^24 points to p, e, cs in cgs: 1.62 -> 1.11-1.16 ms.  Four blocks an
 // SM (128 registers) spill: 1.58 ms.
 template <bool S>
 __global__ void __launch_bounds__(128, 3) k_helm_eos(HelmTable H, long long n, const double* __restrict__ rho,

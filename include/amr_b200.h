@@ -331,8 +331,8 @@ int amr_set_wait_limit(amr_ctx* ctx, int polls);
  * amr_config.persistent_solve > 0. */
 int amr_set_solve_layout(amr_ctx* ctx, int layout, int blocks_per_sm);
 /* The persistent solve's shared-memory relaxation loops as its block 0 sees
- * them (that block holds a brick of every level): ms[0..3] = time waiting
- * for the neighbours' passes, computing passes (ghosts and sweeps), waiting
+ * them (that block holds a brick of every level): ms[0..3] = time fetching
+ * ghosts (waiting for the neighbours' passes included), sweeping, waiting
  * for the loop decision, publishing; the passes and Jacobi sweeps it
  * computed.  Accumulated since the context started. */
 int amr_solve_relax_split(amr_ctx* ctx, double* ms, long long* passes, long long* sweeps);
