@@ -194,7 +194,8 @@ def default_reference():
 
 def build(reference=None, variants=("g05", "zr", "ppm", "ztwd", "ztwd12")):
     reference = reference or default_reference()
-    if not os.path.isdir(reference):
+    # an empty directory stands for an absent tree
+    if not os.path.isdir(reference) or not os.listdir(reference):
         print("[oracle] reference tree not present; using prebuilt oracle/_ref binaries")
         return []
     os.makedirs(REF_OUT, exist_ok=True)
