@@ -190,10 +190,19 @@ int rebuild_topology(amr_ctx* c) {
             if (nd->child[ch] && nd->child[ch]->nchildren() > 0 && nd->child[ch]->level <= maxl) refined++;
         c->h_refined[nd->slot] = refined;
         if (nd->nchildren() > 0 && refined == 0) starts.push_back(nd->slot);
-        for (int f = 0; f < 6; f++)
-            if (c->h_ftype[6 * nd->slot + f] == FACE_AMR && nd->parent && ((nd->cidx >> (f >> 1)) & 1) == (f & 1) &&
-                c->h_ftype[6 * nd->parent->slot + f] == FACE_AMR)
-                c->ghost_chain = true;
+        // a coarse-fine face's bw ghosts and their slopes read the parent's
+        // cells lo..hi along the face's axis (ghost_cell): those past the
+        // parent's interior, on the face's side where the brick touches it
+        // and on the other one where an octant is narrower than the stencil
+        // (4^3 bricks with bw >= 3), must not be coarse-fine ghosts themselves
+        for (int f = 0; f < 6; f++) {
+            if (c->h_ftype[6 * nd->slot + f] != FACE_AMR || !nd->parent) continue;
+            const int ax = f >> 1;
+            const int first = nd->off[ax] - 2 * nd->parent->off[ax] + ((f & 1) ? gnx - bw : 0);
+            const int lo = first / 2 - 1, hi = (first + bw - 1) / 2 + 1;
+            const int* pt = &c->h_ftype[6 * nd->parent->slot + 2 * ax];
+            if ((lo < bw && pt[0] == FACE_AMR) || (hi >= gnx - bw && pt[1] == FACE_AMR)) c->ghost_chain = true;
+        }
     }
     // pack slot lists: all | level 0..maxl | parents 0..maxl | starts
     std::vector<int> packed;

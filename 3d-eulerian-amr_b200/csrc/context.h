@@ -47,7 +47,7 @@ struct amr_ctx {
     int* d_slots = nullptr;                     // all_slots | level lists | parent lists
     std::vector<int> off_all, off_level, off_parent;
     int off_starts = 0, n_starts = 0;           // in d_slots: bricks whose children are all leaves
-    // some coarse-fine ghost reads a coarse-fine ghost (never under proper nesting)
+    // some coarse-fine ghost reads a coarse-fine ghost (under proper nesting only in 4^3 bricks with bw >= 3)
     bool ghost_chain = false;
     amr::RefluxItem* d_reflux = nullptr;
     std::vector<int> off_reflux;

@@ -50,9 +50,12 @@ __device__ __forceinline__ void cell_load(const double* U, int ucount, int gnx, 
 // Cell (x, y, z) (GNX frame, at most one coordinate outside the interior) of
 // brick b.  DEPTH bounds the coarse-fine hops: a coarse-fine ghost reads the
 // parent's cells, whose ghosts across the same face are same-level or domain
-// ghosts under proper nesting, so DEPTH = 1 suffices; a deeper chain sets
-// *err bit 1 (and gives 0) where err is given.  BW, GNX: the brick's sizes
-// where they are known at compile time, else 0.
+// ghosts under proper nesting, so DEPTH = 1 suffices unless the stencil is
+// wider than an octant (4^3 bricks with bw >= 3) and reads the parent's ghosts
+// on its other side.  A deeper chain sets *err bit 1 (and gives 0) where err
+// is given; callers that give none must know that the tree has none
+// (amr_ctx::ghost_chain).  BW, GNX: the brick's sizes where they are known at
+// compile time, else 0.
 template <int DEPTH, int BW, int GNX>
 __device__ __forceinline__ void ghost_cell(const Geom& g, const BrickTable& bt, const double* U, int b, int x, int y,
                                            int z, Cell6& u, int* err) {

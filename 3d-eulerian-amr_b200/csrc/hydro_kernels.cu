@@ -101,8 +101,9 @@ __global__ void k_ghost_fill(Geom g, BrickTable bt, DevState st, const int* __re
 
 // The same for every level in one launch: every ghost value is computed from
 // interior cells (ghost_cell), so no level waits for another.  Needs a tree
-// whose coarse-fine ghosts read no coarse-fine ghosts (proper nesting; the
-// host checks, and runs the level-ordered fill otherwise).  A launch of a
+// whose coarse-fine ghosts read no coarse-fine ghosts (the host looks at
+// every such stencil, amr_ctx::ghost_chain, and runs the level-ordered fill
+// otherwise: proper nesting alone is not enough for 4^3 bricks).  A launch of a
 // small level is 5 us of latency; one per level was 18 to 21% of a step.
 // grid = (bricks, 6 faces); neighbouring threads on neighbouring cells; the
 // brick's sizes at compile time (0: at run time) for the index divisions.
