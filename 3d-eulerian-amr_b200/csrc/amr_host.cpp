@@ -245,9 +245,13 @@ int rebuild_topology(amr_ctx* c) {
     c->off_reflux[maxl + 1] = (int)items.size();
     c->off_reflux_dir[3 * (maxl + 1)] = (int)items.size();
     c->off_rstart = (int)items.size();
+    c->reflux_by_level = false;
     for (int l = maxl; l >= 0; l--)
         for (const RefluxItem& it : c->reflux[l])
-            if (c->h_fixes[6 * it.child + outer_face(it, it.ic)] == 0) items.push_back(it);
+            if (c->h_fixes[6 * it.child + outer_face(it, it.ic)] == 0)
+                items.push_back(it);
+            else if (it.coarse != c->h_parent[it.child])  // k_reflux's climb does not come here
+                c->reflux_by_level = true;
     c->n_rstart = (int)items.size() - c->off_rstart;
     // physical (non-mirror) domain faces for the multipole boundary tables
     {
@@ -395,6 +399,16 @@ int rebuild_topology(amr_ctx* c) {
     c->topo_dirty = false;
     c->topo_version++;  // captured graphs embed the slot lists: rebuild them
     return AMR_OK;
+}
+
+void correct_fluxes(amr_ctx* c, cudaStream_t s) {
+    if (!c->reflux_by_level) {
+        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_rstart, c->n_rstart, c->d_fixes, c->d_rdone, s);
+        return;
+    }
+    for (int l = c->tree.prm.max_level; l >= 0; l--)
+        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_reflux[l], c->off_reflux[l + 1] - c->off_reflux[l],
+                      nullptr, nullptr, s);
 }
 
 }  // namespace amr
@@ -878,8 +892,7 @@ int amr_compute_fluxes(amr_ctx* c) {
     }
     {
         ProfScope ps_(c->prof, KC_REFLUX, c->stream);
-        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_rstart, c->n_rstart, c->d_fixes, c->d_rdone,
-                      c->stream);
+        correct_fluxes(c, c->stream);
     }
     return check_launch(c);
 }

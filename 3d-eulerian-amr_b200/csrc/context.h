@@ -55,6 +55,9 @@ struct amr_ctx {
     // the flux corrections' one launch: its starting items (behind the items
     // in d_reflux), items that correct each face, counters
     int off_rstart = 0, n_rstart = 0;
+    // a corrected face has a reader besides the parent (trees that are not
+    // properly nested): one launch per coarse level
+    bool reflux_by_level = false;
     unsigned char* d_fixes = nullptr;  // [6 cap]
     unsigned* d_rdone = nullptr;       // [6 cap], zero between launches
     std::vector<unsigned char> h_fixes;
@@ -122,6 +125,8 @@ int zt_ready(amr_ctx* c);  // ZTWD context has its EOS (ztwd_host.cpp)
 int zt_check(amr_ctx* c);  // reads and clears the EOS-failure word
 int rebuild_topology(amr_ctx* c);
 int alloc_slot(amr_ctx* c);
+// the coarse-fine corrections of the face fluxes, every level
+void correct_fluxes(amr_ctx* c, cudaStream_t s);
 void graph_release(amr_ctx* c);
 // the plain solve's V-cycle loop in one launch where that can be made (graph_host.cpp)
 int solve_on_device(amr_ctx* c, double tol, int max_cycles, double* l1_error, int* cycles, bool* done);

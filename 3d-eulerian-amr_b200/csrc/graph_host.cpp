@@ -418,7 +418,7 @@ int rec_step(amr_ctx* c, cudaStream_t s, double tol) {
     for (int rk = 0; rk < 3; rk++) {
         TRY(rec_enforce_boundaries(c, s));
         launch_flux(c->geom, c->st, all(c), nall(c), s);
-        launch_reflux(c->geom, c->bt, c->st, c->d_reflux + c->off_rstart, c->n_rstart, c->d_fixes, c->d_rdone, s);
+        correct_fluxes(c, s);
         launch_add_difs(c->geom, c->st, all(c), nall(c), c->bt.h, 0.0, betas[rk], 1, c->tree.root()->slot, c->d_fo, s,
                         dtp);
         launch_phi_time(c->geom, c->st, all(c), nall(c), rk == 0 ? 0 : (rk == 1 ? 2 : 1), s);

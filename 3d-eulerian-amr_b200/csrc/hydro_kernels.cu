@@ -158,7 +158,11 @@ __global__ void __launch_bounds__(FluxBlock<LARGE>::THREADS, FluxBlock<LARGE>::P
 // last of the items that correct the coarse brick's face, goes on to the item
 // that reads that face (a counter per brick face, back to zero for the next
 // launch); no block waits.  fixes[6 slot + face] = items that correct the
-// face.  One block per starting item, thread per (field, face cell).
+// face.  One block per starting item, thread per (field, face cell).  The
+// climb knows one reader of a corrected face, the parent's item.  In a loaded
+// tree that is not properly nested the parent's neighbour can read it too:
+// there (host: reflux_by_level) fixes is null, a block does its item only,
+// and the launches are one per coarse level, finest first.
 // ---------------------------------------------------------------------------
 __global__ void k_reflux(Geom g, BrickTable bt, DevState st, const RefluxItem* __restrict__ items,
                          const unsigned char* __restrict__ fixes, unsigned* done) {
@@ -188,6 +192,7 @@ __global__ void k_reflux(Geom g, BrickTable bt, DevState st, const RefluxItem* _
             Fp[flux_index(it.dir, nx, it.i0 - bw, j0, k0)] = v;
         }
         // the face just corrected, if it is an outer one, and who reads it
+        if (!fixes) return;
         if (it.i0 != bw && it.i0 != gnx - bw) return;
         const int p = it.coarse, side = it.i0 == bw ? 0 : 1, face = 2 * it.dir + side;
         if (bt.parent[p] < 0 || bt.ftype[6 * p + face] == FACE_SIB) return;

@@ -18,7 +18,7 @@ void launch_flux(const Geom& g, const DevState& st, const int* slots, int n, cud
 void launch_flux_f32(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s);
 // every level: items = those whose child's face no item corrects; fixes[6
 // slot + face] = items that correct a face, done[6 slot + face] zero between
-// launches
+// launches; with null fixes the items given and no others (one coarse level)
 void launch_reflux(const Geom& g, const BrickTable& bt, const DevState& st, const RefluxItem* items, int n,
                    const unsigned char* fixes, unsigned* done, cudaStream_t s);
 // with the root's flow-off; dtp: when non-null the step is read from device
