@@ -51,9 +51,10 @@ __host__ __device__ constexpr int recon_reach() { return R == 1 ? 2 : 1; }
 constexpr int PENCIL_PARTS = 3;
 // Register budgets of the kernels: 4^3 and 8^3 bricks' blocks of at most 192
 // threads three to an SM (113 registers), 12^3 bricks' blocks of 432 one (151).
+// THREADS is whole warps, as the CFL kernel is launched (its 432 are 448).
 template <bool LARGE>
 struct FluxBlock {
-    static constexpr int THREADS = PENCIL_PARTS * (LARGE ? 144 : 64), PER_SM = LARGE ? 1 : 3;
+    static constexpr int THREADS = (PENCIL_PARTS * (LARGE ? 144 : 64) + 31) / 32 * 32, PER_SM = LARGE ? 1 : 3;
 };
 
 // Shared memory of a block, [field][cell of the pencil][pencil] with the
