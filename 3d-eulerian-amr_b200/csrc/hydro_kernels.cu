@@ -142,10 +142,11 @@ __global__ void __launch_bounds__(128) k_ghost_fill_all(Geom g, BrickTable bt, D
 // minmod-theta (reconstruct.cpp:60-71) or PPM (reconstruct.cpp:22-58)
 // reconstruction (flux_kernel.cuh).  grid = (bricks, 3 directions)
 // ---------------------------------------------------------------------------
-template <int R, bool LARGE>
-__global__ void __launch_bounds__(FluxBlock<LARGE>::THREADS, FluxBlock<LARGE>::PER_SM) k_flux(Geom g, DevState st, const int* __restrict__ slots) {
+template <int R, FluxBricks B>
+__global__ void __launch_bounds__(FluxBlock<B>::THREADS, FluxBlock<B>::PER_SM)
+    k_flux(Geom g, DevState st, const int* __restrict__ slots, int group) {
     extern __shared__ double flux_smem[];
-    flux_staged<double, R>(g, st, slots[blockIdx.x], flux_smem);
+    flux_staged<double, R, B>(g, st, slots[blockIdx.x], flux_smem, group);
 }
 
 // ---------------------------------------------------------------------------
@@ -424,18 +425,18 @@ __device__ __forceinline__ void store_block_max(double lam, double* out) {
 }
 // grid = (bricks, 3 directions): staged pencils (flux_kernel.cuh), threads
 // rounded up to whole warps
-template <int R, bool LARGE>
-__global__ void __launch_bounds__(FluxBlock<LARGE>::THREADS, FluxBlock<LARGE>::PER_SM)
-    k_max_dt(Geom g, DevState st, const int* __restrict__ slots, double* __restrict__ lam_out) {
+template <int R, FluxBricks B>
+__global__ void __launch_bounds__(FluxBlock<B>::THREADS, FluxBlock<B>::PER_SM)
+    k_max_dt(Geom g, DevState st, const int* __restrict__ slots, double* __restrict__ lam_out, int group) {
     extern __shared__ double flux_smem[];
     const int b = slots[blockIdx.x], d = blockIdx.y;
     double lam;
     if (d == 0)
-        lam = max_eigen_staged<0, R>(g, st, b, flux_smem);
+        lam = max_eigen_staged<0, R, B>(g, st, b, flux_smem, group);
     else if (d == 1)
-        lam = max_eigen_staged<1, R>(g, st, b, flux_smem);
+        lam = max_eigen_staged<1, R, B>(g, st, b, flux_smem, group);
     else
-        lam = max_eigen_staged<2, R>(g, st, b, flux_smem);
+        lam = max_eigen_staged<2, R, B>(g, st, b, flux_smem, group);
     store_block_max(lam, lam_out + 3 * b + d);
 }
 
@@ -502,20 +503,32 @@ void launch_ghost_fill_all(const Geom& g, const BrickTable& bt, const DevState& 
     launch_k(k, dim3(n, 6), 128, 0, s, g, bt, st, slots);
 }
 namespace {
-template <int R, bool LARGE>
+template <int R, FluxBricks B>
 void flux_fp64(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
-    const size_t smem = staged_smem<double, R>(g);
+    const int group = pencil_group<double, R>(g);
+    const size_t smem = staged_smem<double, R>(g, group);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute((const void*)k_flux<R, LARGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_k(k_flux<R, LARGE>, dim3(n, 3), PENCIL_PARTS * g.nx * g.nx, smem, s, g, st, slots);
+        cudaFuncSetAttribute((const void*)k_flux<R, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_k(k_flux<R, B>, dim3(n, 3), PENCIL_PARTS * group, smem, s, g, st, slots, group);
 }
-template <int R, bool LARGE>
+template <int R>
+void flux_fp64(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
+    (g.nx <= 8 ? flux_fp64<R, UP_TO_8> : g.nx == 12 ? flux_fp64<R, OF_12> : flux_fp64<R, IN_GROUPS>)(g, st, slots, n, s);
+}
+template <int R, FluxBricks B>
 void max_dt_fp64(const Geom& g, const DevState& st, const int* slots, int n, double* lam, cudaStream_t s) {
-    const size_t smem = staged_smem<double, R>(g);
+    const int group = pencil_group<double, R>(g);
+    const size_t smem = staged_smem<double, R>(g, group);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute((const void*)k_max_dt<R, LARGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int threads = (PENCIL_PARTS * g.nx * g.nx + 31) / 32 * 32;
-    launch_k(k_max_dt<R, LARGE>, dim3(n, 3), threads, smem, s, g, st, slots, lam);
+        cudaFuncSetAttribute((const void*)k_max_dt<R, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int threads = (PENCIL_PARTS * group + 31) / 32 * 32;
+    launch_k(k_max_dt<R, B>, dim3(n, 3), threads, smem, s, g, st, slots, lam, group);
+}
+template <int R>
+void max_dt_fp64(const Geom& g, const DevState& st, const int* slots, int n, double* lam, cudaStream_t s) {
+    (g.nx <= 8    ? max_dt_fp64<R, UP_TO_8>
+     : g.nx == 12 ? max_dt_fp64<R, OF_12>
+                  : max_dt_fp64<R, IN_GROUPS>)(g, st, slots, n, lam, s);
 }
 }  // namespace
 void launch_flux(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
@@ -523,9 +536,9 @@ void launch_flux(const Geom& g, const DevState& st, const int* slots, int n, cud
     if (g.flux32)
         launch_flux_f32(g, st, slots, n, s);
     else if (g.recon == RECON_PPM)
-        (g.nx > 8 ? flux_fp64<RECON_PPM, true> : flux_fp64<RECON_PPM, false>)(g, st, slots, n, s);
+        flux_fp64<RECON_PPM>(g, st, slots, n, s);
     else
-        (g.nx > 8 ? flux_fp64<RECON_MINMOD, true> : flux_fp64<RECON_MINMOD, false>)(g, st, slots, n, s);
+        flux_fp64<RECON_MINMOD>(g, st, slots, n, s);
 }
 void launch_reflux(const Geom& g, const BrickTable& bt, const DevState& st, const RefluxItem* items, int n,
                    const unsigned char* fixes, unsigned* done, cudaStream_t s) {
@@ -553,9 +566,9 @@ void launch_prolong(const Geom& g, const BrickTable& bt, const DevState& st, con
 void launch_max_dt(const Geom& g, const DevState& st, const int* slots, int n, double* lam, cudaStream_t s) {
     if (n <= 0) return;
     if (g.recon == RECON_PPM)
-        (g.nx > 8 ? max_dt_fp64<RECON_PPM, true> : max_dt_fp64<RECON_PPM, false>)(g, st, slots, n, lam, s);
+        max_dt_fp64<RECON_PPM>(g, st, slots, n, lam, s);
     else
-        (g.nx > 8 ? max_dt_fp64<RECON_MINMOD, true> : max_dt_fp64<RECON_MINMOD, false>)(g, st, slots, n, lam, s);
+        max_dt_fp64<RECON_MINMOD>(g, st, slots, n, lam, s);
 }
 void launch_refine_flags(const Geom& g, const DevState& st, const int* slots, int n, double thr,
                          unsigned char* flags, cudaStream_t s) {

@@ -7,19 +7,26 @@
 
 namespace amr {
 
-template <int R>
-__global__ void __launch_bounds__(FluxBlock<true>::THREADS, 2) k_flux_f32(Geom g, DevState st, const int* __restrict__ slots) {
+template <int R, FluxBricks B>
+__global__ void __launch_bounds__(FluxBlock<OF_12>::THREADS, 2)
+    k_flux_f32(Geom g, DevState st, const int* __restrict__ slots, int group) {
     extern __shared__ float flux_smem_f32[];
-    flux_staged<float, R>(g, st, slots[blockIdx.x], flux_smem_f32);
+    flux_staged<float, R, B>(g, st, slots[blockIdx.x], flux_smem_f32, group);
 }
 
 namespace {
+// one instance for bricks up to 12^3, whose pencils are staged at once
+template <int R, FluxBricks B>
+void flux_fp32(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
+    const int group = pencil_group<float, R>(g);
+    const size_t smem = staged_smem<float, R>(g, group);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute((const void*)k_flux_f32<R, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    launch_k(k_flux_f32<R, B>, dim3(n, 3), PENCIL_PARTS * group, smem, s, g, st, slots, group);
+}
 template <int R>
 void flux_fp32(const Geom& g, const DevState& st, const int* slots, int n, cudaStream_t s) {
-    const size_t smem = staged_smem<float, R>(g);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute((const void*)k_flux_f32<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_k(k_flux_f32<R>, dim3(n, 3), PENCIL_PARTS * g.nx * g.nx, smem, s, g, st, slots);
+    (g.nx <= 12 ? flux_fp32<R, OF_12> : flux_fp32<R, IN_GROUPS>)(g, st, slots, n, s);
 }
 }  // namespace
 
