@@ -22,7 +22,7 @@
 //  * the FP64 sum (its last stages dependent 64-bit shuffles and adds, 500
 //    to 1100 cycles) is formed for the last sweep only.  Before it the loop
 //    compares an integer sum: every thread's squares scaled so that the
-//    first sweep's sum, formed in FP32, is 2^30, cut to a whole number, and
+//    first sweep's sum, formed in FP32, is 2^22, cut to a whole number, and
 //    added with one integer warp reduction per stage.  Unless that sum is
 //    above the threshold by more than its error bound
 //    (RELAX_CLEARLY_ABOVE), the FP64 sums are formed and decide, so every
@@ -166,21 +166,28 @@ __device__ __forceinline__ bool above_half(double resid, double resid0) {
 }
 
 // The integer sum that answers above_half(resid, resid0) for most sweeps: q
-// is the sum over the brick of floor(sum over a thread's cells of
-// (s tmp0)^2) in FP32, with s = 2^15 / sqrt(r), r the first sweep's sum of
-// squares formed in FP32, so that 2^30 stands for resid0 and 2^29 for the
-// threshold.  Errors, in units of the 2^30: r carries one rounding each of a
-// value, its square and at most 5 + 10 additions, 18 x 2^-24; s those of the
-// reciprocal square root (2 ulp) and a product, twice in the square; a value,
-// its product, square and K - 1 <= 5 additions one each: together below
-// 36 x 2^-24 of the sum or 1152 near the threshold; the cuts take off less
-// than one for each of at most 864 threads.  The FP64 sums are within 2^-40.
-// So a q more than 4096 above 2^29 means that the FP64 sum is above half of
-// resid0 as well.  (Ghost faces stay fixed during the sweeps, so the sum does
-// not grow from sweep to sweep and q stays below 2^31; an r outside
+// is the sum over the brick's threads of floor(min(f, RELAX_CLEARLY_ABOVE + 1)),
+// f the sum over a thread's cells of (s tmp0)^2 in FP32, with s =
+// RELAX_SCALE / sqrt(r), r the first sweep's sum of squares formed in FP32, so
+// that 2^22 stands for resid0 and 2^21 for the threshold.  Errors, in units of
+// the 2^22: r carries one rounding each of a value, its square and at most
+// 5 + 10 additions, 18 x 2^-24; s those of the reciprocal square root (2 ulp)
+// and a product, twice in the square; a value, its product, square and
+// K - 1 <= 5 additions one each: together below 36 x 2^-24 of the sum or 5
+// near the threshold; the cuts take off less than one for each of at most 864
+// threads.  The FP64 sums are within 2^-40.  So a q more than 1024 above 2^21
+// means that the FP64 sum is above half of resid0 as well, and one more than
+// 1024 below that it is below.  The minimum changes neither: a thread that it
+// cuts short is above the threshold by itself, and so is q.  It keeps q below
+// 864 (2^21 + 1025) < 2^31: in exact arithmetic the sum does not grow from
+// sweep to sweep (the ghost faces stay fixed), but where a brick's values are
+// at rounding level it can, by any factor.  (A finite first sweep stays
+// finite: later values are bounded by the same cells'.  An r outside
 // [1e-28, 1e28], where FP32 under- or overflows of single squares could
 // matter, takes the FP64 sums in every sweep.)
-constexpr unsigned RELAX_CLEARLY_ABOVE = (1u << 29) + 4096u;
+constexpr float RELAX_SCALE = 2048.0f;
+constexpr unsigned RELAX_HALF = 1u << 21, RELAX_MARGIN = 1024u;
+constexpr unsigned RELAX_CLEARLY_ABOVE = RELAX_HALF + RELAX_MARGIN, RELAX_CLEARLY_BELOW = RELAX_HALF - RELAX_MARGIN;
 
 // The FP64 sum of squares of the values tmp0[r] of every thread's cells:
 // group partials, a barrier, and the pairwise sum in every thread.  Cell t's
@@ -307,7 +314,7 @@ __device__ __forceinline__ double relax_sweeps_in(unsigned x, unsigned y, RelaxS
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) r0 += __shfl_xor_sync(0xffffffffu, r0, o);
     const bool scaled = r0 >= 1.0e-28f && r0 <= 1.0e28f;  // so resid0 is neither 0 nor infinite nor NaN
-    const float s = scaled ? 32768.0f * rsqrtf(r0) : 0.0f;
+    const float s = scaled ? RELAX_SCALE * rsqrtf(r0) : 0.0f;
     bool exact0 = !scaled;  // resid0 is formed: at once, or when a decision asks for it
     double resid0 = exact0 ? relax_sum<NX, TH, CT>(sm, lt, first, sync) : 0.0;
     double resid = resid0;
@@ -321,6 +328,7 @@ __device__ __forceinline__ double relax_sweeps_in(unsigned x, unsigned y, RelaxS
                 const float t = float(tmp0[r]) * s;
                 f += t * t;
             }
+            f = fminf(f, float(RELAX_CLEARLY_ABOVE + 1));  // no 32-bit sum can wrap
             const unsigned part = __reduce_add_sync(0xffffffffu, __float2uint_rz(f));
             if (lane == 0) sm.qred[iters & 1][wp] = part;
             sync();
@@ -329,7 +337,7 @@ __device__ __forceinline__ double relax_sweeps_in(unsigned x, unsigned y, RelaxS
             if (q > RELAX_CLEARLY_ABOVE && iters < 16) continue;
             resid = relax_sum<NX, TH, CT>(sm, lt, tmp0, sync);
             // far enough below the threshold, or the last sweep allowed
-            if ((scaled && q < (1u << 30) - RELAX_CLEARLY_ABOVE) || iters >= 16) break;
+            if ((scaled && q < RELAX_CLEARLY_BELOW) || iters >= 16) break;
             if (!exact0) {
                 sync();  // the sums' scratch is free again
                 resid0 = relax_sum<NX, TH, CT>(sm, lt, first, sync);
