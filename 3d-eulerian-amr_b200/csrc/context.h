@@ -112,6 +112,7 @@ struct amr_ctx {
     int zt_first_solve = 1;  // BinaryDriver::solve's first_call (binary_driver.cpp:297-301)
     amr::Profiler prof;
     struct GraphState* gs = nullptr;  // captured step/solve graphs (graph_host.cpp)
+    long long no_room_version = -1;   // topology at which solve_on_device found no room for its buffers
 
     amr_ctx(const amr::TreeParams& p) : tree(p) {}
 };

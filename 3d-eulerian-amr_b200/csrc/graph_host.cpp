@@ -79,7 +79,7 @@ struct GraphState {
     GridBarrier* d_bar = nullptr;
     unsigned long long* d_tsnap = nullptr;  // [2][cap][6][nx][nx] tagged face snapshots, tsnap_words words an entry
     unsigned long long* d_tpres = nullptr;  // [2][cap][2] tagged per-brick relaxation sums
-    bool persistent_ready = false;  // the buffers below and the launch shape above are set
+    bool persistent_ready = false;  // the buffers around here and the launch shape above are set
     double* d_phikeep = nullptr;  // phi before a plain solve on the device (solve_on_device)
     cudaEvent_t ev_ps[2] = {nullptr, nullptr};  // around the last persistent launch
     double ps_ms_total = 0.0;                   // persistent launches of amr_graph_solve: device time, count
@@ -94,14 +94,13 @@ struct GraphState {
 
 namespace {
 
-// Buffers and launch shape of the persistent solve.  A context that asks for
+// Makes the buffers and launch shape of the persistent solve.  A context that asks for
 // it (amr_config.persistent_solve > 0) starts with layout 0 and that many
 // blocks per SM; the plain solve's own use (solve_on_device) takes the layout
 // that the autotuner keeps on the reference's configurations: 864 threads and
 // one block per SM for 12^3 bricks, 512 threads and two for 8^3.
-int ensure_persistent(amr_ctx* c) {
+int make_persistent(amr_ctx* c) {
     GraphState* g = c->gs;
-    if (g->persistent_ready) return AMR_OK;
     const bool asked = c->cfg.persistent_solve > 0;
     g->layout = !asked && c->geom.nx == 12 ? 1 : 0;
     g->per_sm = asked ? c->cfg.persistent_solve : c->geom.nx == 12 ? 1 : 2;
@@ -114,22 +113,49 @@ int ensure_persistent(amr_ctx* c) {
     if (asked)
         for (int l = 0; l < solve_layouts(c->geom.nx); l++)
             g->pnest_blocks = std::max(g->pnest_blocks, solve_persistent_blocks(c->geom.nx, c->geom.precision, 0, l));
-    if (!g->d_pres3) CUDA_TRY(cudaMalloc(&g->d_pres3, sizeof(double) * 3 * (size_t)c->cap));
-    if (!g->d_pnest) CUDA_TRY(cudaMalloc(&g->d_pnest, sizeof(double) * (size_t)g->pnest_blocks * c->cap));
-    if (!g->d_bar) CUDA_TRY(cudaMalloc(&g->d_bar, sizeof(GridBarrier)));
-    if (!g->d_tsnap) CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap));
-    if (!g->d_tpres) CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
-    for (cudaEvent_t& e : g->ev_ps)
-        if (asked && !e) CUDA_TRY(cudaEventCreate(&e));
-    if (!asked && !g->d_phikeep) CUDA_TRY(cudaMalloc(&g->d_phikeep, sizeof(double) * (size_t)c->cap * c->geom.pnx3));
+    CUDA_TRY(cudaMalloc(&g->d_pres3, sizeof(double) * 3 * (size_t)c->cap));
+    CUDA_TRY(cudaMalloc(&g->d_pnest, sizeof(double) * (size_t)g->pnest_blocks * c->cap));
+    CUDA_TRY(cudaMalloc(&g->d_bar, sizeof(GridBarrier)));
+    CUDA_TRY(cudaMalloc(&g->d_tsnap, sizeof(unsigned long long) * 2 * tsnap_words(c) * (size_t)c->cap));
+    CUDA_TRY(cudaMalloc(&g->d_tpres, sizeof(unsigned long long) * 4 * (size_t)c->cap));
+    if (asked)
+        for (cudaEvent_t& e : g->ev_ps) CUDA_TRY(cudaEventCreate(&e));
+    else
+        CUDA_TRY(cudaMalloc(&g->d_phikeep, sizeof(double) * (size_t)c->cap * c->geom.pnx3));
+    return AMR_OK;
+}
+
+void release_persistent(GraphState* g) {
+    void* bufs[] = {g->d_pres3, g->d_pnest, g->d_bar, g->d_tsnap, g->d_tpres, g->d_phikeep};
+    for (void* p : bufs)
+        if (p) cudaFree(p);
+    g->d_pres3 = g->d_pnest = g->d_phikeep = nullptr;
+    g->d_bar = nullptr;
+    g->d_tsnap = g->d_tpres = nullptr;
+    for (cudaEvent_t& e : g->ev_ps) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    g->persistent_ready = false;
+}
+
+// All of it or, with an error, none of it: a half-made state must not be
+// found by a later call, nor keep memory from one that is short of it.
+int ensure_persistent(amr_ctx* c) {
+    GraphState* g = c->gs;
+    if (g->persistent_ready) return AMR_OK;
+    const int rc = make_persistent(c);
+    if (rc) {
+        release_persistent(g);
+        cudaGetLastError();  // the failed call is reported here, not at the next launch
+        return rc;
+    }
     g->persistent_ready = true;
     return AMR_OK;
 }
 
-int ensure_state(amr_ctx* c) {
-    if (c->gs) return AMR_OK;
-    GraphState* g = new GraphState;
-    c->gs = g;
+int make_state(amr_ctx* c) {
+    GraphState* g = c->gs;
     CUDA_TRY(cudaMalloc(&g->d_ctl, sizeof(Control)));
     CUDA_TRY(cudaMemsetAsync(g->d_ctl, 0, sizeof(Control), c->stream));
     CUDA_TRY(cudaMallocHost(&g->h_ctl, sizeof(Control)));
@@ -151,6 +177,18 @@ int ensure_state(amr_ctx* c) {
     }
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return AMR_OK;
+}
+
+// All or none, as above.
+int ensure_state(amr_ctx* c) {
+    if (c->gs) return AMR_OK;
+    c->gs = new GraphState;
+    const int rc = make_state(c);
+    if (rc) {
+        graph_release(c);
+        cudaGetLastError();
+    }
+    return rc;
 }
 
 int max_level_present(amr_ctx* c) {
@@ -542,13 +580,21 @@ int solve_on_device(amr_ctx* c, double tol, int max_cycles, double* l1_error, in
     // a profiled solve is timed kernel class by kernel class; a context that
     // runs its graph forms persistently has its launch shape for them
     if (c->prof.on || c->cfg.persistent_solve || max_cycles < 1 || (c->geom.nx != 8 && c->geom.nx != 12)) return AMR_OK;
+    // where its buffers found no room they are asked for again after the next
+    // regrid, not in every solve
+    if (c->no_room_version == c->topo_version) return AMR_OK;
     const std::string err0 = c->err;
     auto not_here = [&]() {
         cudaGetLastError();
         c->err = err0;
         return AMR_OK;
     };
-    if (ensure_state(c) != AMR_OK || ensure_persistent(c) != AMR_OK) return not_here();
+    const bool had_state = c->gs;
+    if (ensure_state(c) != AMR_OK || ensure_persistent(c) != AMR_OK) {
+        if (!had_state) graph_release(c);
+        c->no_room_version = c->topo_version;
+        return not_here();
+    }
     GraphState* g = c->gs;
     const size_t bytes = sizeof(double) * (size_t)maxslot(c) * c->geom.pnx3;
     CUDA_TRY(cudaMemcpyAsync(g->d_phikeep, c->st.phi, bytes, cudaMemcpyDeviceToDevice, c->stream));
@@ -591,14 +637,7 @@ void graph_release(amr_ctx* c) {
     if (g->d_nest) cudaFree(g->d_nest);
     if (g->d_snap) cudaFree(g->d_snap);
     if (g->d_counter) cudaFree(g->d_counter);
-    if (g->d_pres3) cudaFree(g->d_pres3);
-    if (g->d_pnest) cudaFree(g->d_pnest);
-    if (g->d_bar) cudaFree(g->d_bar);
-    if (g->d_phikeep) cudaFree(g->d_phikeep);
-    if (g->d_tsnap) cudaFree(g->d_tsnap);
-    if (g->d_tpres) cudaFree(g->d_tpres);
-    for (cudaEvent_t e : g->ev_ps)
-        if (e) cudaEventDestroy(e);
+    release_persistent(g);
     delete g;
     c->gs = nullptr;
 }
