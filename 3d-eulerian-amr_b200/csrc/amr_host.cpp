@@ -28,13 +28,17 @@ thread_local long long amr::g_launch_tally = 0;
         }                                                                                               \
     } while (0)
 
-#define NEED_DEVICE(c)                                                                   \
-    do {                                                                                 \
-        if (!(c)) return AMR_ERR_ARG;                                                    \
-        if (!(c)->has_device) {                                                          \
-            (c)->err = "context has no device pool (created with max_bricks == 0)";      \
-            return AMR_ERR_NODEVICE;                                                     \
-        }                                                                                \
+#define NEED_DEVICE(c)                               \
+    do {                                             \
+        if (!(c)) return AMR_ERR_ARG;                \
+        if (int rc__ = device_ready(c)) return rc__; \
+    } while (0)
+
+// for calls that touch no brick
+#define NEED_POOL(c)                              \
+    do {                                          \
+        if (!(c)) return AMR_ERR_ARG;             \
+        if (int rc__ = has_pool(c)) return rc__;  \
     } while (0)
 
 #define TRY(x)               \
@@ -77,6 +81,11 @@ int rebuild_topology(amr_ctx* c) {
     c->order = T.dfs_order();
     const int n = (int)c->order.size();
     for (int i = 0; i < n; i++) c->order[i]->dfs = i;
+    // a brick without a slot has no place in any table: the tree can be looked
+    // at, but nothing is built for it, on the host or the device
+    c->over_capacity = false;
+    for (Node* nd : c->order) c->over_capacity |= c->has_device && nd->slot < 0;
+    if (c->over_capacity) return device_ready(c);
     const int maxl = T.prm.max_level;
     c->all_slots.resize(n);
     c->level_slots.assign(maxl + 1, {});
@@ -487,15 +496,6 @@ int ensure_stage(amr_ctx* c, size_t count) {
     return dev_alloc(c, &c->d_stage, c->stage_cap);
 }
 
-int check_slots(amr_ctx* c) {
-    for (Node* nd : c->order)
-        if (nd->slot < 0) {
-            c->err = "brick pool exhausted: raise amr_config.max_bricks";
-            return AMR_ERR_CAPACITY;
-        }
-    return AMR_OK;
-}
-
 }  // namespace
 
 namespace amr {
@@ -698,8 +698,7 @@ int amr_init_root(amr_ctx* c) {
     c->tree.init_root();
     c->pending_new.clear();
     c->time = 0.0;
-    TRY(rebuild_topology(c));
-    return check_slots(c);
+    return rebuild_topology(c);
 }
 
 int amr_load_tree(amr_ctx* c, int n, const int* level, const int* loc, const int* age) {
@@ -730,8 +729,7 @@ int amr_load_tree(amr_ctx* c, int n, const int* level, const int* loc, const int
         stack.push_back(ch);
     }
     c->pending_new.clear();
-    TRY(rebuild_topology(c));
-    return check_slots(c);
+    return rebuild_topology(c);
 }
 
 int amr_num_bricks(const amr_ctx* c) { return c ? (int)c->order.size() : 0; }
@@ -769,8 +767,7 @@ int amr_refine_from_flags(amr_ctx* c, const unsigned char* flags, int clear, int
     c->pending_new.clear();
     const bool rc = c->tree.check_for_refine(fl, clear != 0, c->time);
     if (changed) *changed = rc ? 1 : 0;
-    TRY(finish_refine(c));
-    return check_slots(c);
+    return finish_refine(c);
 }
 
 int amr_set_time(amr_ctx* c, double t) {
@@ -812,21 +809,21 @@ int amr_download_state(amr_ctx* c, double* U) {
 }
 
 int amr_get_flow_off(amr_ctx* c, double* fo) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     CUDA_TRY(cudaMemcpyAsync(fo, c->d_fo, sizeof(double) * c->geom.nf, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return AMR_OK;
 }
 
 int amr_set_flow_off(amr_ctx* c, const double* fo) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     CUDA_TRY(cudaMemcpyAsync(c->d_fo, fo, sizeof(double) * c->geom.nf, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return AMR_OK;
 }
 
 int amr_synchronize(amr_ctx* c) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return AMR_OK;
 }
@@ -1155,27 +1152,27 @@ static const char* kClassNames[amr::KC_COUNT] = {
     "source", "phys_boundary", "coarse_correction", "phi_time", "other", "fused_substep"};
 
 int amr_get_stream(amr_ctx* c, void** stream) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     if (!stream) return AMR_ERR_ARG;
     *stream = (void*)c->stream;
     return AMR_OK;
 }
 
 int amr_profile_enable(amr_ctx* c, int on) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     c->prof.collect();
     c->prof.on = on != 0;
     return AMR_OK;
 }
 
 int amr_profile_reset(amr_ctx* c) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     c->prof.reset();
     return AMR_OK;
 }
 
 int amr_profile_get(amr_ctx* c, int cls, double* ms, long long* launches, const char** name) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     if (cls < 0 || cls >= amr::KC_COUNT) return AMR_ERR_ARG;
     c->prof.collect();
     if (ms) *ms = c->prof.ms[cls];
@@ -1191,7 +1188,7 @@ int amr_launch_count(amr_ctx* c, long long* kernels) {
 }
 
 int amr_profile_units(amr_ctx* c, int cls, long long* units) {
-    NEED_DEVICE(c);
+    NEED_POOL(c);
     if (cls < 0 || cls >= amr::KC_COUNT || !units) return AMR_ERR_ARG;
     c->prof.collect();
     *units = c->prof.units[cls];

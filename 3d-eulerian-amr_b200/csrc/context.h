@@ -18,6 +18,7 @@ struct amr_ctx {
     std::string err;
     double time = 0.0;
     bool has_device = false;
+    bool over_capacity = false;  // the tree has more bricks than the pool: no call may run on it
     cudaStream_t stream = nullptr;
 
     // device pool
@@ -121,6 +122,20 @@ namespace amr {
 inline bool is_ztwd(const amr_ctx* c) { return c->cfg.physics == AMR_PHYSICS_ZTWD; }
 inline bool has_gravity(const amr_ctx* c) {
     return c->cfg.physics == AMR_PHYSICS_EULER_GRAVITY || c->cfg.physics == AMR_PHYSICS_ZTWD;
+}
+inline int has_pool(amr_ctx* c) {
+    if (c->has_device) return AMR_OK;
+    c->err = "context has no device pool (created with max_bricks == 0)";
+    return AMR_ERR_NODEVICE;
+}
+// AMR_OK where device calls may run on the tree: a pool, and a slot for every brick
+inline int device_ready(amr_ctx* c) {
+    if (int rc = has_pool(c)) return rc;
+    if (c->over_capacity) {
+        c->err = "brick pool exhausted: raise amr_config.max_bricks";
+        return AMR_ERR_CAPACITY;
+    }
+    return AMR_OK;
 }
 int zt_ready(amr_ctx* c);  // ZTWD context has its EOS (ztwd_host.cpp)
 int zt_check(amr_ctx* c);  // reads and clears the EOS-failure word

@@ -283,10 +283,7 @@ __global__ void k_m1m2(Geom g, BrickTable bt, DevState st, const int* __restrict
 // per-brick moments of one field, in DFS order
 int moments(amr_ctx* c, int field, int mode, std::vector<double>& per) {
     if (!c) return AMR_ERR_ARG;
-    if (!c->has_device) {
-        c->err = "context has no device pool";
-        return AMR_ERR_NODEVICE;
-    }
+    TRY(device_ready(c));
     if (field < 0 || field >= c->geom.nf) return AMR_ERR_ARG;
     const int n = (int)c->order.size();
     std::vector<double> h3(n);
@@ -493,10 +490,7 @@ int amr_m1m2data(amr_ctx* c, double* out, double* l1) {
         c->err = "M1M2data needs the ZTWD state";
         return AMR_ERR_ARG;
     }
-    if (!c->has_device) {
-        c->err = "context has no device pool";
-        return AMR_ERR_NODEVICE;
-    }
+    TRY(device_ready(c));
     return m1m2data(c, out, l1);
 }
 

@@ -551,7 +551,7 @@ void count_replay(amr_ctx* c, long long top_kernels) {
 
 int need(amr_ctx* c) {
     if (!c) return AMR_ERR_ARG;
-    if (!c->has_device) return AMR_ERR_NODEVICE;
+    TRY(device_ready(c));
     if (!has_gravity(c)) {
         c->err = "graph solve needs a self-gravitating context";
         return AMR_ERR_ARG;

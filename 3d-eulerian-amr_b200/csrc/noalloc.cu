@@ -80,10 +80,7 @@ extern "C" {
 int amr_poisson_boundaries_noalloc(amr_ctx* c) {
     using namespace amr;
     if (!c) return AMR_ERR_ARG;
-    if (!c->has_device) {
-        c->err = "context has no device pool";
-        return AMR_ERR_NODEVICE;
-    }
+    if (int rc = device_ready(c)) return rc;
     if (!has_gravity(c)) {
         c->err = "Poisson call on a context created without self-gravity";
         return AMR_ERR_ARG;

@@ -45,10 +45,7 @@ int check_launch(amr_ctx* c) {
 
 int need_gravity(amr_ctx* c) {
     if (!c) return AMR_ERR_ARG;
-    if (!c->has_device) {
-        c->err = "context has no device pool";
-        return AMR_ERR_NODEVICE;
-    }
+    TRY(device_ready(c));
     if (!has_gravity(c)) {
         c->err = "Poisson call on a context created without self-gravity";
         return AMR_ERR_ARG;

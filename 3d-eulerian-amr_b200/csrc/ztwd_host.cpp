@@ -33,10 +33,7 @@ namespace amr {
 
 int zt_ready(amr_ctx* c) {
     if (!c) return AMR_ERR_ARG;
-    if (!c->has_device) {
-        c->err = "context has no device pool";
-        return AMR_ERR_NODEVICE;
-    }
+    TRY(device_ready(c));
     if (!is_ztwd(c)) {
         c->err = "ZTWD call on a context created without AMR_PHYSICS_ZTWD";
         return AMR_ERR_ARG;
