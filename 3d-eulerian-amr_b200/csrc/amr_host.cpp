@@ -1070,6 +1070,10 @@ int amr_fused_sub_step(amr_ctx* c, double dt, double beta, int blocks_per_sm) {
         c->err = "fused substep: minmod reconstruction with bw 2 only";
         return AMR_ERR_ARG;
     }
+    if (c->geom.nx != 8) {  // the kernel's index arithmetic is that of 12^3 cells
+        c->err = "fused substep: bricks of 8^3 only";
+        return AMR_ERR_ARG;
+    }
     TRY(fused_setup(c));
     CUDA_TRY(cudaMemsetAsync(c->d_fctl, 0, sizeof(unsigned int) * 2, c->stream));
     FusedArgs a{};

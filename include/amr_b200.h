@@ -148,7 +148,8 @@ int amr_state_max(amr_ctx* ctx, int field, double* vmax);
 /* ---- driver sequences ----------------------------------------------------- */
 /* HydroDriver::sub_step (euler/hydro_driver.cpp:200-214). */
 int amr_sub_step(amr_ctx* ctx, double dt, double beta);
-/* amr_sub_step (Euler physics without gravity) as one persistent launch:
+/* amr_sub_step (Euler physics without gravity; minmod, bw 2, bricks of 8^3) as
+ * one persistent launch:
  * ghost zones computed where needed, fluxes (FP32 in the mixed form),
  * coarse-fine corrections and the RK combination per brick, finest level
  * first; the result goes to a second state array that then becomes the
