@@ -1017,17 +1017,34 @@ namespace {
 
 // Work list (finest level first, depth-first within a level) and publish
 // masks of the fused substep, rebuilt when the topology changes.
+int make_fused(amr_ctx* c) {
+    const size_t cap = c->cap;
+    CUDA_TRY(cudaMalloc(&c->d_U1, sizeof(double) * cap * c->geom.ucount));
+    CUDA_TRY(cudaMemcpyAsync(c->d_U1, c->st.U, sizeof(double) * cap * c->geom.ucount, cudaMemcpyDeviceToDevice,
+                             c->stream));
+    CUDA_TRY(cudaMalloc(&c->d_pubmask, cap));
+    CUDA_TRY(cudaMalloc(&c->d_pub, sizeof(double) * cap * 6 * c->geom.nf * c->geom.nx * c->geom.nx));
+    CUDA_TRY(cudaMalloc(&c->d_fdone, sizeof(int) * cap));
+    CUDA_TRY(cudaMemsetAsync(c->d_fdone, 0, sizeof(int) * cap, c->stream));
+    CUDA_TRY(cudaMalloc(&c->d_fctl, sizeof(unsigned int) * 2));
+    return AMR_OK;
+}
+
 int fused_setup(amr_ctx* c) {
     const int cap = c->cap;
     if (!c->d_U1) {
-        CUDA_TRY(cudaMalloc(&c->d_U1, sizeof(double) * (size_t)cap * c->geom.ucount));
-        CUDA_TRY(cudaMemcpyAsync(c->d_U1, c->st.U, sizeof(double) * (size_t)cap * c->geom.ucount,
-                                 cudaMemcpyDeviceToDevice, c->stream));
-        CUDA_TRY(cudaMalloc(&c->d_pubmask, (size_t)cap));
-        CUDA_TRY(cudaMalloc(&c->d_pub, sizeof(double) * (size_t)cap * 6 * c->geom.nf * c->geom.nx * c->geom.nx));
-        CUDA_TRY(cudaMalloc(&c->d_fdone, sizeof(int) * (size_t)cap));
-        CUDA_TRY(cudaMemsetAsync(c->d_fdone, 0, sizeof(int) * (size_t)cap, c->stream));
-        CUDA_TRY(cudaMalloc(&c->d_fctl, sizeof(unsigned int) * 2));
+        const int rc = make_fused(c);
+        if (rc) {  // none of them rather than some: d_U1 says that all are there
+            void* bufs[] = {c->d_U1, c->d_pubmask, c->d_pub, c->d_fdone, c->d_fctl};
+            for (void* p : bufs)
+                if (p) cudaFree(p);
+            c->d_U1 = c->d_pub = nullptr;
+            c->d_pubmask = nullptr;
+            c->d_fdone = nullptr;
+            c->d_fctl = nullptr;
+            cudaGetLastError();
+            return rc;
+        }
     }
     if (c->fused_version == c->topo_version) return AMR_OK;
     std::vector<int2> work;

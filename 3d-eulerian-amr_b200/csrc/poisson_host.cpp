@@ -21,6 +21,7 @@ using namespace amr;
     do {                                                                                      \
         cudaError_t e__ = (call);                                                             \
         if (e__ != cudaSuccess) {                                                             \
+            cudaGetLastError(); /* reported here, not at the next launch */                   \
             c->err = std::string("CUDA error: ") + cudaGetErrorString(e__) + " at " + #call; \
             return AMR_ERR_CUDA;                                                              \
         }                                                                                     \
@@ -50,13 +51,15 @@ int need_gravity(amr_ctx* c) {
         c->err = "Poisson call on a context created without self-gravity";
         return AMR_ERR_ARG;
     }
-    if (!c->d_bphi) {
-        const size_t nb = (size_t)c->cap * 6 * c->geom.pnx * c->geom.pnx;
-        CUDA_TRY(cudaMalloc(&c->d_bphi, sizeof(double) * nb));
-        CUDA_TRY(cudaMemsetAsync(c->d_bphi, 0, sizeof(double) * nb, c->stream));
-        CUDA_TRY(cudaMalloc(&c->d_pres, sizeof(double) * c->cap));
-        CUDA_TRY(cudaMalloc(&c->d_perr, sizeof(int) * 2));
+    if (!c->d_bphi) {  // the last of the buffers made: all are there when it is
+        const size_t nb = sizeof(double) * (size_t)c->cap * 6 * c->geom.pnx * c->geom.pnx;
+        double* bphi = nullptr;
+        if (!c->d_pres) CUDA_TRY(cudaMalloc(&c->d_pres, sizeof(double) * c->cap));
+        if (!c->d_perr) CUDA_TRY(cudaMalloc(&c->d_perr, sizeof(int) * 2));
         CUDA_TRY(cudaMemsetAsync(c->d_perr, 0, sizeof(int) * 2, c->stream));
+        CUDA_TRY(cudaMalloc(&bphi, nb));
+        c->d_bphi = bphi;
+        CUDA_TRY(cudaMemsetAsync(c->d_bphi, 0, nb, c->stream));
     }
     return AMR_OK;
 }
