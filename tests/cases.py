@@ -3,6 +3,7 @@
 import os
 
 import numpy as np
+import pytest
 
 from conftest import GOLDEN
 
@@ -59,7 +60,8 @@ def live_initial_state(variant, args, workdir, table_path=None):
     from dumpio import read_dump
 
     exe = ref_binary(variant)
-    assert exe is not None, "oracle/_ref/%s_harness is needed for this case" % variant
+    if exe is None:
+        pytest.skip("reference oracle binary not built (oracle/build_ref.py): %s_harness" % variant)
     if table_path is not None:
         os.symlink(table_path, os.path.join(workdir, "helmholtz.table"))
     out = os.path.join(workdir, "init.bin")
