@@ -50,8 +50,10 @@ template <int R>
 __host__ __device__ constexpr int recon_reach() { return R == 1 ? 2 : 1; }
 constexpr int PENCIL_PARTS = 3;
 // Which bricks an instance is for, and its register budget: 4^3 and 8^3 ones
-// in blocks of at most 192 threads, three to an SM; 12^3 ones in blocks of 432,
-// one to an SM; larger ones in groups of at most 64 pencils, one group after
+// in blocks of at most 192 threads, three to an SM (96 registers: of the 18
+// warps five share a quarter of the SM; fluxes spill 256 bytes with minmod, 612
+// with PPM, the PPM eigenvalues 528); 12^3 ones in blocks of 432, one to an SM
+// (128 registers, PPM fluxes spill 116 bytes); larger ones in groups of at most 64 pencils, one group after
 // the other in a block of 192 (all of a 16^3 brick's pencils would be 768
 // threads and 247 KB).  THREADS is whole warps, as the CFL kernel is launched
 // (its 432 are 448).

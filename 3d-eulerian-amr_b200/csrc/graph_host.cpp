@@ -681,9 +681,9 @@ int amr_solve_phase_waits(amr_ctx* c, double* wait_ms, int n, double* level_sum_
 }
 
 // The shared-memory relaxation loops of the persistent solve as block 0
-// sees them (its brick is in every level): ms[0..3] = waiting for the
-// neighbours' passes, computing passes, waiting for the loop decision,
-// publishing; the passes and the Jacobi sweeps block 0 computed.
+// sees them (its brick is in every level): ms[0..3] = fetching ghosts (waiting
+// for the neighbours' passes included), sweeping, waiting for the loop
+// decision, publishing; the passes and the Jacobi sweeps block 0 computed.
 int amr_solve_relax_split(amr_ctx* c, double* ms, long long* passes, long long* sweeps) {
     if (!c || !ms || !passes || !sweeps) return AMR_ERR_ARG;
     if (!c->gs) {

@@ -196,7 +196,8 @@ void launch_helm_invert(const HelmTable& H, long long n, const double* rho, cons
                         const double* abar, const double* zbar, int from_entropy, double* T, double* p, double* e,
                         double* cs, double* cv, double* s, int* iters, int* status, cudaStream_t st) {
     if (n <= 0) return;
-    // the warps that fit at once share the points, a whole warp's at least
+    // the warps that fit at once (148 SMs, three blocks of four warps each)
+    // share the points, a whole warp's at least
     const long long warps = 148LL * 3 * 4, per_warp = std::max(32LL, (n + warps - 1) / warps);
     const int blocks = (int)((n + 4 * per_warp - 1) / (4 * per_warp));
     const auto k = s || from_entropy ? k_helm_invert<true> : k_helm_invert<false>;

@@ -47,7 +47,9 @@ __device__ __forceinline__ void fused_wait(const FusedArgs& A, int child) {
 // threads take the faces in two full rounds; 256 left a third round with a
 // quarter of them.  Faces are numbered so that neighbouring threads read and
 // write neighbouring words in every direction (with the pencil fastest in x,
-// two thirds of the shared-memory wavefronts were bank conflicts).
+// two thirds of the shared-memory wavefronts were bank conflicts).  Two blocks
+// an SM are 18 warps, five on a quarter of it: 96 registers, 160 bytes of
+// spills in FP64.
 constexpr int FUSED_BLOCK = 288;
 constexpr int CROSS = 512 + 6 * 2 * 64;  // interior + ghost slabs
 constexpr int FACES = 9 * 64;            // faces of one direction

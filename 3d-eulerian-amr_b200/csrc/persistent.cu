@@ -82,9 +82,9 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, unsigned& target, un
 // Block layout of the solve for bricks of NX^3 interior cells: TPB threads
 // per block, NX^3 / TPB cells per thread in the relaxation (every layout
 // gives the same results bit for bit).  With 8^3 bricks and 512 threads a
-// block relaxes two bricks at once (one per half) on levels with more
-// bricks than blocks, so it holds two staged bricks; the other layouts take
-// such levels brick by brick.  MINB: blocks per SM the registers are
+// block relaxes two bricks at once (one per half) on levels with more bricks
+// than the shared-memory loop takes, so it holds two staged bricks; the other
+// layouts take such levels brick by brick.  MINB: blocks per SM the registers are
 // budgeted for.  resb: the bricks one block can hold in the shared-memory
 // relaxation loop, as many as leave room for MINB blocks per SM (three
 // buffers and dphi1 each: 28 KB for an 8^3 brick in FP64, 80 KB for a 12^3

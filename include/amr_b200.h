@@ -324,10 +324,10 @@ int amr_relax_passes(amr_ctx* ctx, long long* per_level, int n);
 int amr_set_wait_limit(amr_ctx* ctx, int polls);
 /* Block layout of the persistent solve kernel (no reference counterpart:
  * the reference has no kernels): layout 0 .. count-1 of the brick size
- * (8^3: 512 threads, one cell each, two bricks per block on levels with
- * more bricks than blocks; 256 threads, two cells each.  12^3: 576 threads,
- * three cells each; 864, two; 288, six) and the blocks per SM of the launch
- * (0: as many as fit).  Every layout gives the same results bit for bit.
+ * (8^3: 512 threads, one cell each, two bricks at once on levels with more
+ * bricks than the blocks hold in shared memory; 256 threads, two cells each.
+ * 12^3: 576 threads, three cells each; 864, two; 288, six) and the blocks per
+ * SM of the launch (0: as many as fit).  Every layout gives the same results bit for bit.
  * The captured graphs are re-captured at their next call.  Needs
  * amr_config.persistent_solve > 0. */
 int amr_set_solve_layout(amr_ctx* ctx, int layout, int blocks_per_sm);
