@@ -458,9 +458,10 @@ class AMR:
         return ms
 
     def solve_relax_split(self):
-        """Block 0's view of the shared-memory relaxation loops: ms waiting
-        for neighbours, computing, waiting for the decision, publishing;
-        passes and sweeps."""
+        """Block 0's view of the shared-memory relaxation loops: ms fetching
+        ghosts (waits for the neighbours' passes included; wait_neighbours_ms),
+        sweeping (pass_ms), waiting for the decision, publishing; passes and
+        sweeps."""
         ms = np.zeros(4)
         p, s = ctypes.c_longlong(), ctypes.c_longlong()
         self._check(self.lib.amr_solve_relax_split(self.ctx, _dptr(ms), ctypes.byref(p), ctypes.byref(s)))

@@ -88,7 +88,7 @@ BYTES_PER_BRICK = {
 # (7.93 GB of algorithmic bytes).  The solve's arrays stay in L2 across its
 # V-cycles, so DRAM sees the cold fill, the per-launch zeroing of the tagged
 # relaxation buffers and the dirty write-back.
-ZT_SOLVE_DRAM_BYTES_PER_LAUNCH = {8: 16.69e6, 12: 185.0e6}
+ZT_SOLVE_DRAM_BYTES_PER_LAUNCH = {8: 11.70e6, 12: 178.8e6}
 
 
 # the keys of the roofline object on the bench line (the rest of the solve's
@@ -293,7 +293,8 @@ def aggregate(ms_total, cells, world, dist, device="cuda"):
 def run_form(amr, ini, form, args, world, local, torch, dist, e2e=False, profile=False):
     """Build the workload and time K steps of one form of our path.
 
-    form: "fp64"  plain FP64, host-orchestrated (reference operation order)
+    form: "fp64"  plain FP64: one launch per hydro operation, one per solve's
+                  V-cycle loop (the bits of the reference's operation order)
           "graph" FP64, whole RK3 step replayed from a captured CUDA graph with
                   every loop decided on the device (bitwise equal to fp64)
           "persistent" the graph form with each solve's V-cycle loop as one
