@@ -703,30 +703,45 @@ int amr_init_root(amr_ctx* c) {
 
 int amr_load_tree(amr_ctx* c, int n, const int* level, const int* loc, const int* age) {
     if (!c || n <= 0 || !level || !loc) return AMR_ERR_ARG;
-    c->tree.init_root();
     if (level[0] != 0) return AMR_ERR_ARG;
-    std::vector<Node*> stack{c->tree.root()};
-    if (age) c->tree.root()->age = age[0];
+    // the whole list is looked at before the present tree goes: a refused
+    // list leaves it as it is
+    struct Open {  // a node whose descendants are being listed
+        int loc[3];
+        unsigned children;
+    };
+    std::vector<Open> open{{{0, 0, 0}, 0u}};  // open[l]: the one of level l
+    std::vector<int> octant(n, 0);
     for (int i = 1; i < n; i++) {
-        while (!stack.empty() && stack.back()->level >= level[i]) stack.pop_back();
-        if (stack.empty() || stack.back()->level != level[i] - 1) {
+        if (level[i] < 1 || level[i] > (int)open.size()) {
             c->err = "amr_load_tree: list is not a depth-first pre-order";
             return AMR_ERR_ARG;
         }
-        Node* p = stack.back();
-        int cidx = 0;
+        open.resize(level[i]);
+        Open& p = open.back();
         for (int d = 0; d < 3; d++) {
-            const int bit = loc[3 * i + d] - 2 * p->loc[d];
+            const int bit = loc[3 * i + d] - 2 * p.loc[d];
             if (bit != 0 && bit != 1) {
                 c->err = "amr_load_tree: location is not a child of the preceding node";
                 return AMR_ERR_ARG;
             }
-            cidx |= bit << d;
+            octant[i] |= bit << d;
         }
-        if (p->child[cidx]) return AMR_ERR_ARG;
-        Node* ch = c->tree.create_child(p, cidx);
+        if (p.children & (1u << octant[i])) {
+            c->err = "amr_load_tree: a brick is listed twice";
+            return AMR_ERR_ARG;
+        }
+        p.children |= 1u << octant[i];
+        open.push_back({{loc[3 * i], loc[3 * i + 1], loc[3 * i + 2]}, 0u});
+    }
+    c->tree.init_root();
+    std::vector<Node*> path{c->tree.root()};
+    if (age) c->tree.root()->age = age[0];
+    for (int i = 1; i < n; i++) {
+        path.resize(level[i]);
+        Node* ch = c->tree.create_child(path.back(), octant[i]);
         if (age) ch->age = age[i];
-        stack.push_back(ch);
+        path.push_back(ch);
     }
     c->pending_new.clear();
     return rebuild_topology(c);
